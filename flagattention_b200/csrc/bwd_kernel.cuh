@@ -483,12 +483,13 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
           if constexpr (MODE == MODE_Q) {
             keep_bits = row < args.M ? mk[static_cast<int64_t>(col0 >> 5) * args.M + row] : 0u;
           } else {
-            // the warp's 32 key rows share one word index; lane c fetches query col0 + c's word (bit l =
-            // key l of the warp), and a 32 x 32 bit transpose across the warp (five butterfly steps)
-            // leaves in lane l the word whose bit c is the decision for (key l, query col0 + c)
+            // the warp's 32 key rows share one word index; lane c fetches the word of query
+            // col0 + keep_index_of(c) (bit l = key keep_index_of(l) of the warp), and a 32 x 32 bit transpose
+            // across the warp (five butterfly steps) leaves in lane l the word of key keep_index_of(l) with the
+            // queries in the order of keep_bit_of(); one more shuffle brings every lane its own key's word
             const int wi = (r0 + (warp & 3) * 32) >> 5;
-            keep_bits = (col0 + lane < args.M && wi < args.drop.mask_words)
-                            ? mk[static_cast<int64_t>(wi) * args.M + col0 + lane] : 0u;
+            const int query = col0 + keep_index_of(lane);
+            keep_bits = (query < args.M && wi < args.drop.mask_words) ? mk[static_cast<int64_t>(wi) * args.M + query] : 0u;
 #pragma unroll
             for (int s = 16; s >= 1; s >>= 1) {
               const uint32_t m = s == 16 ? 0x0000ffffu : s == 8 ? 0x00ff00ffu : s == 4 ? 0x0f0f0f0fu
@@ -496,6 +497,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
               const uint32_t y = __shfl_xor_sync(0xffffffffu, keep_bits, s);
               keep_bits = (lane & s) ? ((keep_bits & ~m) | ((y >> s) & m)) : ((keep_bits & m) | ((y << s) & ~m));
             }
+            keep_bits = __shfl_sync(0xffffffffu, keep_bits, keep_bit_of(lane));
           }
         } else if constexpr (MODE == MODE_Q) {
           keep_bits = dropout_keep_word(args.drop, head_base + static_cast<uint64_t>(row) * args.N + col0);
@@ -580,19 +582,19 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
           } else {
             float dp_a = __uint_as_float(t2[c]);
             float dp_b = __uint_as_float(t2[c + 1]);
-            float pd_a = p_a, pd_b = p_b;
-            if constexpr (DROPOUT) {
-              const bool keep_a = (keep_bits >> c) & 1u;
-              const bool keep_b = (keep_bits >> (c + 1)) & 1u;
-              pd_a = keep_a ? p_a : 0.f;
-              pd_b = keep_b ? p_b : 0.f;
-              dp_a = keep_a ? dp_a * args.drop.inv_keep : 0.f;
-              dp_b = keep_b ? dp_b * args.drop.inv_keep : 0.f;
-            }
             // dS = P * (dP - delta)
+            uint64_t dp2;
+            if constexpr (DROPOUT) {
+              dp_a = __uint_as_float(t2[c] & keep_mask_one(keep_bits, c));
+              dp_b = __uint_as_float(t2[c + 1] & keep_mask_one(keep_bits, c + 1));
+              dp2 = f2_fma(f2_pack(dp_a, dp_b), f2_pack(args.drop.inv_keep, args.drop.inv_keep), ndel2);
+            } else {
+              dp2 = f2_add(f2_pack(dp_a, dp_b), ndel2);
+            }
             float ds_a, ds_b;
-            f2_unpack(f2_mul(f2_pack(p_a, p_b), f2_add(f2_pack(dp_a, dp_b), ndel2)), ds_a, ds_b);
-            t1[c >> 1] = pack2<BF16>(pd_a, pd_b);
+            f2_unpack(f2_mul(f2_pack(p_a, p_b), dp2), ds_a, ds_b);
+            t1[c >> 1] = pack2<BF16>(p_a, p_b);
+            if constexpr (DROPOUT) t1[c >> 1] &= keep_mask_pair(keep_bits, c);
             t2[c >> 1] = pack2<BF16>(ds_a, ds_b);
           }
         }

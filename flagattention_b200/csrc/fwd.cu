@@ -131,6 +131,8 @@ extern "C" int b200attn_fwd(const b200attn_fwd_params* p, void* stream) {
   if (p->dropout_p > 0.f && p->keep_mask != nullptr) {
     a.drop.keep_mask = p->keep_mask;
     a.drop.mask_words = cdiv(p->N, 32);
+    const int rc_mask = launch_keep_mask(a.drop, p->B, p->Hq, p->M, p->N, a.d_min, a.d_max, static_cast<cudaStream_t>(stream));
+    if (rc_mask) return rc_mask;
   }
   a.status = p->status;
   a.n_zblocks = cdiv(p->M, 256);

@@ -63,8 +63,9 @@ typedef struct {
    * q/k pair) and usable as a sliding window. Rows with no visible key give o = 0, lse = -inf. */
   int32_t band, dist_min, dist_max;
   /* Optional (dropout_p > 0): b200attn_keep_mask_bytes() bytes that receive the keep decisions, one
-   * bit per (query, key), for b200attn_bwd to reuse instead of re-evaluating Philox (the reference
-   * recomputes them in both backward kernels, flash.py:660-664,846-850). NULL = not stored. */
+   * bit per (query, key), drawn by a kernel of its own ahead of the forward and for b200attn_bwd to reuse instead
+   * of re-evaluating Philox (the reference recomputes them in both backward kernels, flash.py:660-664,846-850).
+   * The order of the bits is the library's own. NULL = not stored. */
   uint32_t* keep_mask;
 } b200attn_fwd_params;
 
