@@ -56,26 +56,38 @@ int launch_keep_mask(const DropoutCtx& ctx, int B, int H, int M, int N, int d_mi
   return B200ATTN_OK;
 }
 
-// One warp per row of D elements: lanes read 16-byte vectors, shuffle-reduce, lane 0 writes.
+// (-lse * log2e) of one query, the form the backward kernels use. A row without any visible key (lse = -inf) gets
+// -inf like the padding, so that every probability recomputed against it, exp2(s*c + (-inf)), is exactly 0.
+__device__ __forceinline__ float stats_nlse(float lse) {
+  return lse == -INFINITY ? -INFINITY : -lse * 1.4426950408889634f;
+}
+
+// D / 8 lanes per row: 16-byte loads, shuffle-reduce. With `stats` (and then `lse`) the rows run over [0, Mpad) of
+// every head and the kernel also leaves the statistics of each pair of rows, in the layout of stats_kernel (two
+// neighbouring rows sit in one warp), which saves a launch and a pass over lse and delta: the preprocess of a small
+// backward (B2 Hq8 512 x 512 D128) is launch-bound.
 template <int D, int O_KIND, bool DO_BF16>
 __global__ void __launch_bounds__(256)
 delta_kernel(const void* __restrict__ o, const void* __restrict__ d_o, float* __restrict__ delta,
-             int64_t o_sb, int64_t o_sh, int64_t o_sm, int64_t do_sb, int64_t do_sh, int64_t do_sm, int B,
-             int H, int M, float* __restrict__ zero_rows) {
+             int64_t o_sb, int64_t o_sh, int64_t o_sm, int64_t do_sb, int64_t do_sh, int64_t do_sm,
+             int H, int M, float* __restrict__ zero_rows, const float* __restrict__ lse, float4* __restrict__ stats,
+             int Mrows) {
   constexpr int VEC = 8;                 // elements per lane per step
   constexpr int LANES = D / VEC;         // lanes that carry data for one row (2..16)
   constexpr int ROWS_PER_WARP = 32 / LANES;
   const int lane = threadIdx.x & 31;
-  const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int sub = lane / LANES;
   const int col = (lane % LANES) * VEC;
-  const int64_t row_id = static_cast<int64_t>(warp_global) * ROWS_PER_WARP + sub;
-  const int64_t total = static_cast<int64_t>(B) * H * M;
+  // a block takes 8 * ROWS_PER_WARP consecutive rows of one head (no 64-bit division per row)
+  const int blocks_per_head = (Mrows + 8 * ROWS_PER_WARP - 1) / (8 * ROWS_PER_WARP);
+  const int bh = static_cast<int>(blockIdx.x) / blocks_per_head;
+  const int m = (static_cast<int>(blockIdx.x) - bh * blocks_per_head) * (8 * ROWS_PER_WARP) + (threadIdx.x >> 5) * ROWS_PER_WARP + sub;
+  const bool live = m < M;
+  const int64_t row_id = static_cast<int64_t>(bh) * M + m;
   float acc = 0.f;
-  if (row_id < total) {
-    const int m = static_cast<int>(row_id % M);
-    const int h = static_cast<int>((row_id / M) % H);
-    const int b = static_cast<int>(row_id / (static_cast<int64_t>(M) * H));
+  if (live) {
+    const int b = bh / H;
+    const int h = bh - b * H;
     const int64_t o_off = b * o_sb + h * o_sh + m * o_sm + col;
     const int64_t do_off = b * do_sb + h * do_sh + m * do_sm + col;
     float ov[VEC], gv[VEC];
@@ -114,57 +126,64 @@ delta_kernel(const void* __restrict__ o, const void* __restrict__ d_o, float* __
   }
 #pragma unroll
   for (int s = LANES / 2; s >= 1; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-  if (row_id < total && (lane % LANES) == 0) delta[row_id] = acc;
+  if (live && (lane % LANES) == 0) delta[row_id] = acc;
+  if (stats != nullptr) {
+    const float nl = live ? stats_nlse(lse[row_id]) : -INFINITY;
+    const float nl_next = __shfl_down_sync(0xffffffffu, nl, LANES);
+    const float acc_next = __shfl_down_sync(0xffffffffu, acc, LANES);
+    if (m < Mrows && (lane % (2 * LANES)) == 0)  // (Mrows is even: the pair is one head's)
+      stats[(static_cast<int64_t>(bh) * Mrows + m) / 2] = make_float4(nl, nl_next, -acc, -acc_next);
+  }
 }
 
 // Per-query statistics for the backward / total-attention kernels, two queries per float4:
 // stats4[b, h, m/2] = (-lse[m]*log2e, -lse[m+1]*log2e, -delta[m], -delta[m+1]); the padding rows
-// m in [M, Mpad) get (-inf, 0). Rows without any visible key (lse = -inf) also get -inf, so that
-// every probability recomputed against them, exp2(s*c + (-inf)), is exactly 0.
+// m in [M, Mpad) get (-inf, 0). This kernel serves total attention, which has no delta (0 here);
+// the backward's come from delta_kernel.
 __global__ void __launch_bounds__(256)
-stats_kernel(const float* __restrict__ lse, const float* __restrict__ delta, float4* __restrict__ stats,
-             int64_t BH, int M, int Mpad) {
+stats_kernel(const float* __restrict__ lse, float4* __restrict__ stats, int64_t BH, int M, int Mpad) {
   const int half = Mpad / 2;
   const int64_t total = BH * half;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t bh = i / half;
     const int m = static_cast<int>(i - bh * half) * 2;
-    float nl[2] = {-INFINITY, -INFINITY}, nd[2] = {0.f, 0.f};
+    float nl[2] = {-INFINITY, -INFINITY};
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      if (m + j < M) {
-        const float l = lse[bh * M + m + j];
-        nl[j] = (l == -INFINITY) ? -INFINITY : -l * 1.4426950408889634f;
-        nd[j] = delta != nullptr ? -delta[bh * M + m + j] : 0.f;
-      }
+      if (m + j < M) nl[j] = stats_nlse(lse[bh * M + m + j]);
     }
-    stats[i] = make_float4(nl[0], nl[1], nd[0], nd[1]);
+    stats[i] = make_float4(nl[0], nl[1], 0.f, 0.f);
   }
 }
 
-int launch_stats(const float* lse, const float* delta, float2* stats, int B, int H, int M, int Mpad,
-                 cudaStream_t stream) {
+int launch_stats(const float* lse, float2* stats, int B, int H, int M, int Mpad, cudaStream_t stream) {
   const int64_t total = static_cast<int64_t>(B) * H * (Mpad / 2);
   int64_t blocks = (total + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
   stats_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
-      lse, delta, reinterpret_cast<float4*>(stats), static_cast<int64_t>(B) * H, M, Mpad);
+      lse, reinterpret_cast<float4*>(stats), static_cast<int64_t>(B) * H, M, Mpad);
   B200ATTN_CUDA_OK(cudaGetLastError());
   return B200ATTN_OK;
 }
 
 template <int D>
 static int launch_delta(const b200attn_tensor* o, int o_dtype, const b200attn_tensor* d_o, int do_dtype,
-                        float* delta, int B, int H, int M, cudaStream_t stream, float* zero_rows) {
+                        float* delta, int B, int H, int M, cudaStream_t stream, float* zero_rows, const float* lse,
+                        float2* stats, int Mpad) {
   constexpr int ROWS_PER_WARP = 32 / (D / 8);
-  const int64_t total = static_cast<int64_t>(B) * H * M;
-  const int64_t warps = (total + ROWS_PER_WARP - 1) / ROWS_PER_WARP;
-  const unsigned blocks = static_cast<unsigned>((warps + 7) / 8);
+  const int rows = stats != nullptr ? Mpad : M;
+  const int64_t n_blocks = static_cast<int64_t>(B) * H * cdiv(rows, 8 * ROWS_PER_WARP);
+  if (n_blocks > 2147483647ll) {
+    set_error("bwd_delta: too many rows for the grid");
+    return B200ATTN_EINVAL;
+  }
+  const unsigned blocks = static_cast<unsigned>(n_blocks);
 #define B200ATTN_DELTA(OK, DB)                                                                        \
   delta_kernel<D, OK, DB><<<blocks, 256, 0, stream>>>(o->ptr, d_o->ptr, delta, o->stride[0],          \
                                                       o->stride[1], o->stride[2], d_o->stride[0],    \
-                                                      d_o->stride[1], d_o->stride[2], B, H, M, zero_rows)
+                                                      d_o->stride[1], d_o->stride[2], H, M, zero_rows,       \
+                                                      lse, reinterpret_cast<float4*>(stats), rows)
   const bool db = do_dtype == B200ATTN_BF16;
   if (o_dtype == B200ATTN_F32) { if (db) B200ATTN_DELTA(B200ATTN_F32, true); else B200ATTN_DELTA(B200ATTN_F32, false); }
   else if (o_dtype == B200ATTN_BF16) { if (db) B200ATTN_DELTA(B200ATTN_BF16, true); else B200ATTN_DELTA(B200ATTN_BF16, false); }
@@ -300,7 +319,8 @@ extern "C" int b200attn_dropout_mask(uint8_t* mask, int32_t B, int32_t H, int32_
 
 namespace b200attn {
 int bwd_delta(const b200attn_tensor* o, int32_t o_dtype, const b200attn_tensor* d_o, int32_t do_dtype,
-              float* delta, int32_t B, int32_t H, int32_t M, int32_t D, void* stream, float* zero_rows) {
+              float* delta, int32_t B, int32_t H, int32_t M, int32_t D, void* stream, float* zero_rows,
+              const float* lse, float2* stats, int Mpad) {
   if (delta == nullptr || B <= 0 || H <= 0 || M <= 0) {
     set_error("bwd_delta: bad argument");
     return B200ATTN_EINVAL;
@@ -315,10 +335,10 @@ int bwd_delta(const b200attn_tensor* o, int32_t o_dtype, const b200attn_tensor* 
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (D) {
-    case 16: return launch_delta<16>(o, o_dtype, d_o, do_dtype, delta, B, H, M, s, zero_rows);
-    case 32: return launch_delta<32>(o, o_dtype, d_o, do_dtype, delta, B, H, M, s, zero_rows);
-    case 64: return launch_delta<64>(o, o_dtype, d_o, do_dtype, delta, B, H, M, s, zero_rows);
-    case 128: return launch_delta<128>(o, o_dtype, d_o, do_dtype, delta, B, H, M, s, zero_rows);
+    case 16: return launch_delta<16>(o, o_dtype, d_o, do_dtype, delta, B, H, M, s, zero_rows, lse, stats, Mpad);
+    case 32: return launch_delta<32>(o, o_dtype, d_o, do_dtype, delta, B, H, M, s, zero_rows, lse, stats, Mpad);
+    case 64: return launch_delta<64>(o, o_dtype, d_o, do_dtype, delta, B, H, M, s, zero_rows, lse, stats, Mpad);
+    case 128: return launch_delta<128>(o, o_dtype, d_o, do_dtype, delta, B, H, M, s, zero_rows, lse, stats, Mpad);
     default:
       set_error("bwd_delta: head dimension %d not in {16, 32, 64, 128}", D);
       return B200ATTN_EINVAL;
@@ -329,7 +349,7 @@ int bwd_delta(const b200attn_tensor* o, int32_t o_dtype, const b200attn_tensor* 
 extern "C" int b200attn_bwd_delta(const b200attn_tensor* o, int32_t o_dtype, const b200attn_tensor* d_o,
                                   int32_t do_dtype, float* delta, int32_t B, int32_t H, int32_t M,
                                   int32_t D, void* stream) {
-  return b200attn::bwd_delta(o, o_dtype, d_o, do_dtype, delta, B, H, M, D, stream, nullptr);
+  return b200attn::bwd_delta(o, o_dtype, d_o, do_dtype, delta, B, H, M, D, stream, nullptr, nullptr, nullptr, 0);
 }
 
 extern "C" int b200attn_merge_partial(float* o_acc, float* lse_acc, const float* o_part,

@@ -273,9 +273,8 @@ extern "C" int b200attn_bwd_stages(const b200attn_bwd_params* p, void* stream_, 
     float* zero_rows = nullptr;
     if (fused_dq(p->D, stages) && (stages & B200ATTN_BWD_STAGE_KV))
       zero_rows = reinterpret_cast<float*>(stats + static_cast<size_t>(p->B) * p->Hq * pad128(p->M));
-    rc = bwd_delta(&p->o, p->o_dtype, &p->d_o, p->dtype, p->delta, p->B, p->Hq, p->M, p->D, stream_, zero_rows);
-    if (rc) return rc;
-    rc = launch_stats(p->lse, p->delta, stats, p->B, p->Hq, p->M, pad128(p->M), stream);
+    rc = bwd_delta(&p->o, p->o_dtype, &p->d_o, p->dtype, p->delta, p->B, p->Hq, p->M, p->D, stream_, zero_rows,
+                   p->lse, stats, pad128(p->M));
     if (rc) return rc;
   }
   switch (p->D) {
@@ -304,7 +303,7 @@ extern "C" int b200attn_total_attention(const b200attn_total_params* p, void* st
   }
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   float2* stats = static_cast<float2*>(p->workspace);
-  rc = launch_stats(p->lse, nullptr, stats, p->B, p->Hq, p->M, pad128(p->M), stream);
+  rc = launch_stats(p->lse, stats, p->B, p->Hq, p->M, pad128(p->M), stream);
   if (rc) return rc;
   switch (p->D) {
     case 16: return run_total<16>(p, stats, stream);
@@ -371,7 +370,7 @@ extern "C" int b200attn_total_attention_static(const b200attn_total_params* p, v
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   // Every entry the kernel reads ([0, need)) is rewritten here first, so whatever an earlier call
   // left in the array never matters.
-  rc = launch_stats(p->lse, nullptr, stats, p->B, p->Hq, p->M, pad128(p->M), stream);
+  rc = launch_stats(p->lse, stats, p->B, p->Hq, p->M, pad128(p->M), stream);
   if (rc) return rc;
   switch (p->D) {
     case 16: return run_total<16>(p, stats, stream);

@@ -51,13 +51,13 @@ int encode_tmap_4d(CUtensorMap* out, const b200attn_tensor& t, int elem_bytes, i
 // Checks the TMA requirements of one operand; returns 0 or B200ATTN_EINVAL.
 int check_tma_operand(const b200attn_tensor& t, int elem_bytes, const char* name);
 
-// Writes the padded per-query statistics the backward / total-attention kernels stream
-// (aux_kernels.cu). `delta` may be null (total attention).
-// delta[b,h,m] = sum_d o*do; optionally also clears a contiguous fp32 [B, H, M, D] array.
+// delta[b,h,m] = sum_d o*do; optionally also clears a contiguous fp32 [B, H, M, D] array and, with `stats`, writes
+// the padded per-query statistics that the backward kernels stream (aux_kernels.cu).
 int bwd_delta(const b200attn_tensor* o, int32_t o_dtype, const b200attn_tensor* d_o, int32_t do_dtype,
-              float* delta, int32_t B, int32_t H, int32_t M, int32_t D, void* stream, float* zero_rows);
-int launch_stats(const float* lse, const float* delta, float2* stats, int B, int H, int M, int Mpad,
-                 cudaStream_t stream);
+              float* delta, int32_t B, int32_t H, int32_t M, int32_t D, void* stream, float* zero_rows,
+              const float* lse, float2* stats, int Mpad);
+// The statistics alone, with zero deltas (total attention).
+int launch_stats(const float* lse, float2* stats, int B, int H, int M, int Mpad, cudaStream_t stream);
 
 // Smallest integer threshold T such that a Philox word x (folded to [0, 2^31)) is KEPT iff x > T,
 // equivalent to `float(x) * 4.6566127342e-10f > dropout_p` evaluated in fp32.
