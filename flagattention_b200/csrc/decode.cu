@@ -63,6 +63,8 @@ decode_partial_kernel(const DecodeArgs a) {
   const int b = bhk / a.Hkv;
   const int rows = a.groups * a.M;  // <= R
   const bool paged = a.block_table != nullptr;
+  pdl_trigger();
+  pdl_wait();
   const int N = paged ? a.context_lens[b] : a.N;
   const int P_SEQ = N - a.M;
 
@@ -281,13 +283,8 @@ decode_partial_kernel(const DecodeArgs a) {
 
 template <int D, int R>
 int launch_rows(const DecodeArgs& a, bool bf16, unsigned grid, cudaStream_t stream) {
-  if (bf16) {
-    decode_partial_kernel<D, R, true><<<grid, DEC_THREADS, 0, stream>>>(a);
-  } else {
-    decode_partial_kernel<D, R, false><<<grid, DEC_THREADS, 0, stream>>>(a);
-  }
-  B200ATTN_CUDA_OK(cudaGetLastError());
-  return B200ATTN_OK;
+  return launch(CHAINED, bf16 ? decode_partial_kernel<D, R, true> : decode_partial_kernel<D, R, false>, dim3(grid),
+                DEC_THREADS, 0, stream, a);
 }
 
 template <int D>

@@ -180,6 +180,8 @@ splitkv_combine_kernel(const float* __restrict__ part_o, const float* __restrict
   constexpr int CACHED = 1024;
   __shared__ float w_sh[CACHED];
   __shared__ float red[4];
+  pdl_trigger();
+  pdl_wait();
   const int64_t row = blockIdx.x;  // (b*H + h)*M + m
   const int m = static_cast<int>(row % M);
   const int64_t bh = row / M;
@@ -239,17 +241,9 @@ splitkv_combine_kernel(const float* __restrict__ part_o, const float* __restrict
 
 static int launch_splitkv_combine(const b200attn_splitkv_params* p, bool bf16, unsigned rows,
                                   cudaStream_t stream) {
-  if (bf16) {
-    splitkv_combine_kernel<true><<<rows, 128, 0, stream>>>(
-        p->part_o, p->part_lse, p->o.ptr, p->lse, p->o.stride[0], p->o.stride[1], p->o.stride[2], p->Hq,
-        p->M, p->D, p->num_splits);
-  } else {
-    splitkv_combine_kernel<false><<<rows, 128, 0, stream>>>(
-        p->part_o, p->part_lse, p->o.ptr, p->lse, p->o.stride[0], p->o.stride[1], p->o.stride[2], p->Hq,
-        p->M, p->D, p->num_splits);
-  }
-  B200ATTN_CUDA_OK(cudaGetLastError());
-  return B200ATTN_OK;
+  return launch(CHAINED, bf16 ? splitkv_combine_kernel<true> : splitkv_combine_kernel<false>, dim3(rows), 128, 0, stream,
+                p->part_o, p->part_lse, p->o.ptr, p->lse, p->o.stride[0], p->o.stride[1], p->o.stride[2], p->Hq, p->M, p->D,
+                p->num_splits);
 }
 
 }  // namespace b200attn

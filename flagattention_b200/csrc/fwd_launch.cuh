@@ -25,9 +25,7 @@ int launch_fwd_variant(const FwdLaunch& L) {
     return B200ATTN_OK;
   });
   if (rc) return rc;
-  kernel<<<L.grid, 384, smem, L.stream>>>(L.tmQ, L.tmK, L.tmV, L.tmO, L.args);
-  B200ATTN_CUDA_OK(cudaGetLastError());
-  return B200ATTN_OK;
+  return launch(CHAINED, kernel, L.grid, 384, smem, L.stream, L.tmQ, L.tmK, L.tmV, L.tmO, L.args);
 }
 
 template <int D>

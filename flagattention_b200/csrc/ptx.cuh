@@ -36,6 +36,16 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// ------------------------------------------------- overlap with the previous kernel of the stream
+// A kernel that is launched with LaunchForm::chained (common.cuh) may start while its predecessor still runs.
+// pdl_wait() blocks until the predecessor has completed and its writes are visible: every thread calls it before its
+// first access to global memory, also threads that then have nothing to do, because the next kernel in turn relies on
+// this one not completing before its predecessor. pdl_trigger() lets the next kernel start once every block of this
+// one has called it; a kernel that allocates TMEM calls it after the allocation, or a successor's block on the same
+// SM could take the columns and wait for this kernel for ever. Both do nothing in an ordinary launch.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ----------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
