@@ -26,9 +26,9 @@ int launch_bwd_variant(const BwdLaunch& L) {
     return B200ATTN_OK;
   });
   if (rc) return rc;
-  kernel<<<L.grid, BwdSmem<D, MODE, FUSED>::THREADS, smem, L.stream>>>(L.tmA1, L.tmA2, L.tmB1, L.tmB2, L.tmO1, L.tmO2, L.args);
-  B200ATTN_CUDA_OK(cudaGetLastError());
-  return B200ATTN_OK;
+  const LaunchForm form{false, L.args.kv_split > 1 ? static_cast<unsigned>(L.args.kv_split) : 1u};
+  return launch(form, kernel, L.grid, BwdSmem<D, MODE, FUSED>::THREADS, smem, L.stream, L.tmA1, L.tmA2, L.tmB1, L.tmB2, L.tmO1,
+                L.tmO2, L.args);
 }
 
 template <int D>

@@ -25,18 +25,25 @@ int cuda_fail(cudaError_t e, const char* what);
   } while (0)
 
 // How a kernel is launched beyond its grid: `chained`, it may overlap the previous kernel of the stream and calls
-// pdl_wait() (ptx.cuh).
+// pdl_wait() (ptx.cuh); `cluster` consecutive blocks form a cluster.
 struct LaunchForm {
   bool chained = false;
+  unsigned cluster = 1;
 };
 template <class... Params, class... Args>
 inline int launch(const LaunchForm& form, void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem,
                   cudaStream_t stream, const Args&... args) {
-  cudaLaunchAttribute attr[1] = {};
+  cudaLaunchAttribute attr[2] = {};
   unsigned n = 0;
   if (form.chained) {
     attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (form.cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = form.cluster;
+    attr[n].val.clusterDim.y = 1;
+    attr[n++].val.clusterDim.z = 1;
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
@@ -52,7 +59,7 @@ inline int launch(const LaunchForm& form, void (*kernel)(Params...), dim3 grid, 
 // to show, and are launched chained: B1 H4 128 x 128 D64 forward 5.7 -> 4.8 us a call replayed from a graph, paged
 // decode of 32 sequences up to 4096 keys 95.4 -> 92.8 us. The backward's kernels are not: chained, its dK/dV pass runs
 // beside the waiting blocks of the dQ conversion, and a step of B64 H32 512 x 512 D64 took 817 instead of 796 us.
-constexpr LaunchForm CHAINED{true};
+constexpr LaunchForm CHAINED{true, 1};
 
 // One-time set-up per device (kernel attributes, device properties) that any host thread may
 // trigger: `run(f)` executes `f` once for the current device under std::call_once and hands back its
@@ -77,6 +84,9 @@ struct PerDeviceOnce {
 int encode_tmap_4d(CUtensorMap* out, const b200attn_tensor& t, int elem_bytes, int64_t B, int64_t H,
                    int64_t rows, int64_t D, int box_cols, int box_rows, int swizzle,
                    const char* name, int box_heads = 1);
+
+// Multiprocessor count of the current device, looked up once per device.
+int sm_count();
 
 // Checks the TMA requirements of one operand; returns 0 or B200ATTN_EINVAL.
 int check_tma_operand(const b200attn_tensor& t, int elem_bytes, const char* name);
@@ -246,6 +256,7 @@ __device__ __forceinline__ uint32_t dropout_keep_word_strided(const DropoutCtx& 
 
 // ------------------------------------------------------------ small helpers
 __host__ __device__ constexpr int cdiv(int a, int b) { return (a + b - 1) / b; }
+__host__ constexpr int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 template <bool BF16>
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {

@@ -38,12 +38,6 @@ static void make_o_tmap(const b200attn_fwd_params* p, FwdLaunch& L) {
 
 }  // namespace b200attn
 
-namespace b200attn {
-namespace {
-int cached_sm_count();
-}  // namespace
-}  // namespace b200attn
-
 extern "C" int b200attn_fwd(const b200attn_fwd_params* p, void* stream) {
   using namespace b200attn;
   if (p == nullptr) {
@@ -150,7 +144,7 @@ extern "C" int b200attn_fwd(const b200attn_fwd_params* p, void* stream) {
   // enough that one CTA per item, placed by the hardware as SMs fall free, measured 3-7 % faster.
   a.n_items = static_cast<int>(static_cast<int64_t>(p->B) * p->Hq * a.n_zblocks);  // range checked above
   const bool chain = a.causal == 0 || cdiv(p->N, 128) <= 32;
-  const int n_ctas = chain ? cached_sm_count() : a.n_items;
+  const int n_ctas = chain ? sm_count() : a.n_items;
   L.grid = dim3(static_cast<unsigned>(a.n_items < n_ctas ? a.n_items : n_ctas));
   L.bf16 = p->dtype == B200ATTN_BF16;
   L.dropout = p->dropout_p > 0.f;
@@ -493,32 +487,11 @@ extern "C" int b200attn_paged_attention(const b200attn_paged_params* p, void* st
   return run_splitkv(&sp, &pk, stream);
 }
 
-namespace b200attn {
-namespace {
-
-// Multiprocessor count of the current device, looked up once per device.
-int cached_sm_count() {
-  static PerDeviceOnce once;
-  static int counts[PerDeviceOnce::MAX_DEVICES] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= PerDeviceOnce::MAX_DEVICES) return 148;
-  once.run([&]() -> int {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    counts[dev] = n;   // written inside call_once, read only after it has returned
-    return B200ATTN_OK;
-  });
-  return counts[dev];
-}
-
-}  // namespace
-}  // namespace b200attn
-
 extern "C" int b200attn_splitkv_num_splits(int32_t B, int32_t Hq, int32_t Hkv, int32_t M, int32_t N,
                                            int32_t D, int32_t num_sms) {
   using namespace b200attn;
   if (B <= 0 || Hq <= 0 || Hkv <= 0 || M <= 0 || N <= 0 || Hq % Hkv != 0) return 1;
-  if (num_sms <= 0) num_sms = cached_sm_count();
+  if (num_sms <= 0) num_sms = sm_count();
   const int groups = Hq / Hkv;
   const int n_blocks = cdiv(N, 128);
   if (static_cast<int64_t>(groups) * M <= DECODE_MAX_ROWS) {

@@ -106,6 +106,20 @@ int encode_tmap_4d(CUtensorMap* out, const b200attn_tensor& t, int elem_bytes, i
   return B200ATTN_OK;
 }
 
+int sm_count() {
+  static PerDeviceOnce once;
+  static int counts[PerDeviceOnce::MAX_DEVICES] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= PerDeviceOnce::MAX_DEVICES) return 148;
+  once.run([&]() -> int {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    counts[dev] = n;   // written inside call_once, read only after it has returned
+    return B200ATTN_OK;
+  });
+  return counts[dev];
+}
+
 int32_t dropout_keep_threshold(float dropout_p) {
   // Largest x in [0, 2^31) with float(x) * scale <= p, or -1 when every x is kept.
   const float scale = 4.6566127342e-10f;
