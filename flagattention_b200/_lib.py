@@ -162,6 +162,28 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+_HOST = None
+
+
+def host():
+    """The native host path (``csrc/torch_host.cpp``), bound once to the library above. Like the library it has
+    no stand-in: if it was not built, this raises."""
+    global _HOST
+    if _HOST is None:
+        lib = load()
+        try:
+            from . import _host
+        except ImportError as e:
+            raise RuntimeError("flagattention_b200/_host.so is missing or does not load: build it with "
+                               "`python -m flagattention_b200.build`") from e
+        from .status import poll_pointer
+        _host.bind(tuple(ctypes.cast(getattr(lib, name), c_void_p).value for name in (
+            "b200attn_fwd", "b200attn_bwd_stages", "b200attn_bwd_workspace_bytes", "b200attn_fwd_splitkv",
+            "b200attn_splitkv_num_splits", "b200attn_paged_attention", "b200attn_last_error")), poll_pointer)
+        _HOST = _host
+    return _HOST
+
+
 def dtype_code(dtype: torch.dtype) -> int:
     try:
         return _DTYPE_CODE[dtype]

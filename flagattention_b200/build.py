@@ -1,4 +1,5 @@
-"""Builds ``libb200attn.so`` in-tree with nvcc for sm_100a.
+"""Builds ``libb200attn.so`` in-tree with nvcc for sm_100a, and ``_host.so`` (the operators' host path, plain C++
+against torch's headers) with the host compiler.
 
 ``python -m flagattention_b200.build`` compiles every ``csrc/*.cu`` (in parallel, one object per
 file, skipping objects newer than all sources) and links the shared library next to this file.
@@ -10,6 +11,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -17,6 +19,8 @@ PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 OBJ_DIR = CSRC / "build"
 LIB_PATH = PKG_DIR / "libb200attn.so"
+HOST_SRC = CSRC / "torch_host.cpp"
+HOST_PATH = PKG_DIR / "_host.so"     # Python extension module: the operators' host path
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -54,13 +58,33 @@ def _compile_one(src: Path, force: bool, verbose: bool, hdr_mtime: float) -> Pat
     return obj
 
 
+def _build_host(force: bool) -> None:
+    """Compiles the host path against torch's C++ headers and libraries."""
+    newest = max(HOST_SRC.stat().st_mtime, (PKG_DIR.parent / "include" / "b200attn.h").stat().st_mtime)
+    if not force and HOST_PATH.exists() and HOST_PATH.stat().st_mtime > newest:
+        return
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+    cuda_include = Path(_nvcc()).resolve().parent.parent / "include"
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[f"-I{p}" for p in include_paths()], f"-I{cuda_include}", f"-I{sysconfig.get_paths()['include']}",
+           str(HOST_SRC), "-o", str(HOST_PATH), *[f"-L{p}" for p in library_paths()],
+           "-ltorch_python", "-ltorch", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed for {HOST_SRC.name}:\n{res.stdout}\n{res.stderr}")
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     """Compile and link the library; returns its path."""
     OBJ_DIR.mkdir(parents=True, exist_ok=True)
     sources = sorted(CSRC.glob("*.cu"))
     hdr_mtime = _newest_header_mtime()
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 2)) as pool:
+        host = pool.submit(_build_host, force)
         objs = list(pool.map(lambda s: _compile_one(s, force, verbose, hdr_mtime), sources))
+        host.result()
     if force or not LIB_PATH.exists() or any(o.stat().st_mtime > LIB_PATH.stat().st_mtime for o in objs):
         cmd = [_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-o", str(LIB_PATH),
                *[str(o) for o in objs]]

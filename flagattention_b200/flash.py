@@ -121,6 +121,10 @@ def flash_attention_split_kv(q, k, v, causal=False, sm_scale=None):
     """Forward-only attention over split keys/values ("flash decoding"): same arguments, checks and
     result as the reference operator (``split_kv.py:282-347``); the result has ``q``'s dtype
     whatever the split count. Not differentiable, like the reference's."""
+    if q.is_cuda:
+        o = _lib.host().split_kv(q, k, v, causal, sm_scale)  # None: a call that needs a copy first or is to raise
+        if o is not None:
+            return o
     Dq, Dk, Dv = q.shape[-1], k.shape[-1], v.shape[-1]
     assert Dq == Dk == Dv
     assert Dk in _SUPPORTED_HEAD_DIMS
@@ -309,5 +313,11 @@ def flash_attention(q, k, v, causal=False, sm_scale=None, dropout_p=0.0,
             result is the 5-tuple ``(out, log_normalizer|None, total_attention|None, seed|None,
             offset|None)``; otherwise just ``out``.
     """
+    # The ordinary call runs natively from here (csrc/torch_host.cpp); it hands back None for a call that needs a copy
+    # first, is to raise, or runs under a transform.
+    if dropout_p == 0 and not (return_log_normalizer or return_total_attention or return_seed_offset) and q.is_cuda:
+        o = _lib.host().flash(q, k, v, causal, sm_scale)
+        if o is not None:
+            return o
     return FlashAttentionFunction.apply(q, k, v, causal, sm_scale, dropout_p, return_log_normalizer,
                                         return_total_attention, return_seed_offset)

@@ -36,6 +36,11 @@ def paged_attention(query, key_cache, value_cache, context_lens, block_tables, a
             depend on it beyond fp32 rounding).
     Returns ``[num_seqs, num_query_heads, head_size]`` in ``query.dtype``.
     """
+    if query.is_cuda:
+        out = _lib.host().paged(query, key_cache, value_cache, context_lens, block_tables, attn_scale, max_context_len,
+                                num_splits)
+        if out is not None:  # None: a call that needs a conversion first or is to raise
+            return out
     if not (query.is_cuda and key_cache.is_cuda and value_cache.is_cuda):
         raise RuntimeError("paged_attention runs on CUDA tensors only (no CPU fallback)")
     if query.dim() != 3 or key_cache.dim() != 4 or value_cache.shape != key_cache.shape:

@@ -43,6 +43,8 @@ _devices: dict[int, _DeviceStatus] = {}
 def _index(device) -> int:
     if device is None:
         return torch.cuda.current_device()
+    if type(device) is int:
+        return device
     device = torch.device(device)
     return device.index if device.index is not None else torch.cuda.current_device()
 
@@ -101,6 +103,11 @@ def poll(device) -> torch.Tensor:
         st.pending = True
         st.last_poll = now
     return st.word
+
+
+def poll_pointer(index: int) -> int:
+    """``poll`` for the native host path: the address of the word of device ``index``."""
+    return poll(index).data_ptr()
 
 
 def check_device_status(device=None) -> None:
