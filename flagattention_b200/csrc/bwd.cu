@@ -99,7 +99,7 @@ __global__ void dq_convert_kernel(const float* __restrict__ acc, uint16_t* __res
 static int bwd_kv_split(const BwdArgs& a, int D) {
   const int n_z = a.n_zblocks;
   const int64_t pairs = static_cast<int64_t>(a.B) * a.Hkv;
-  const int sms = sm_count();
+  const int sms = sm_count() * (D == 64 || D == 32 ? 2 : 1);  // blocks that run at a time, see BwdSmem::DUO
   if (pairs * n_z >= 4ll * sms) return 1;  // long lists of blocks balance by themselves
   int64_t sum = 0, longest = 0;
   for (int z = 0; z < n_z; ++z) {
@@ -133,7 +133,7 @@ static int bwd_kv_split(const BwdArgs& a, int D) {
 }
 
 // Whether the backward of this head dimension produces dQ inside the dK/dV pass.
-static bool fused_dq(int D, int stages) { return (D == 128 || D == 64) && !(stages & B200ATTN_BWD_STAGE_UNFUSED); }
+static bool fused_dq(int D, int stages) { return D >= 32 && !(stages & B200ATTN_BWD_STAGE_UNFUSED); }
 
 template <int D>
 static int run_bwd(const b200attn_bwd_params* p, float2* stats, cudaStream_t stream, int stages) {
@@ -268,8 +268,8 @@ extern "C" size_t b200attn_bwd_workspace_bytes(int32_t B, int32_t Hq, int32_t Hk
   (void)Hkv; (void)N;
   if (B <= 0 || Hq <= 0 || M <= 0) return 0;
   size_t bytes = static_cast<size_t>(B) * Hq * b200attn::pad128(M) * sizeof(float2);
-  // D = 128 and 64: fp32 dQ accumulator of the fused pass behind the statistics
-  if (D == 128 || D == 64) bytes += static_cast<size_t>(B) * Hq * M * D * sizeof(float);
+  // fp32 dQ accumulator of the fused pass behind the statistics
+  if (b200attn::fused_dq(D, 0)) bytes += static_cast<size_t>(B) * Hq * M * D * sizeof(float);
   return bytes;
 }
 

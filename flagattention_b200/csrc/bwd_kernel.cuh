@@ -16,22 +16,28 @@
 // as in the reference (dV uses the masked P and is scaled by 1/(1-p) at the end; dP is masked and
 // scaled by 1/(1-p) before delta is subtracted).
 //
-// Roles: warps 0-3 and 4-7 are two softmax groups that alternate steps (thread r <-> row r), warp 8
-// issues tcgen05.mma, warp 9 drives TMA. TMEM: accumulators (D columns each) followed by two
+// Roles: warps 0-3 and 4-7 are two softmax groups, each on half of a step's columns (thread r <-> row r);
+// further warps issue tcgen05.mma and drive TMA. TMEM: accumulators (D columns each) followed by two
 // (T1, T2) buffers of 64+64 fp32 columns; P / dS overwrite T1 as packed 16-bit pairs and are
 // consumed from TMEM as the A operand of the accumulating MMAs.
 //
-// FUSED (MODE_KV, D = 128 and 64): the same pass also produces dQ, so P and dS are computed once for
+// FUSED (MODE_KV, D >= 32): the same pass also produces dQ, so P and dS are computed once for
 // the whole backward. The softmax groups leave dS^T a second time in shared memory ([128 keys x 64
 // queries], 128-byte swizzled rows); the MMA warp forms dQ^T = K^T dS^T (A = the resident K tile read
-// MN-major, 128 x 64 fp32) in the step's dead T2 columns (D = 128) or in columns of its own (D = 64),
-// ahead of the step's accumulating products
-// so that the read-back overlaps them; four extra warps read it back, transpose it through two
-// 16 KB staging tiles ([32 queries][128 features] fp32, the layout of the accumulator rows) and add
+// MN-major, 128 x 64 fp32) in the step's dead T2 columns, ahead of the step's accumulating products
+// so that the read-back overlaps them; D / 32 extra warps read it back, transpose it through two
+// staging tiles ([32 queries][D features] fp32, the layout of the accumulator rows) and add
 // it to an fp32 dQ accumulator in global memory with cp.reduce.async.bulk (.add.f32), since every
 // key block contributes to every query row. A conversion kernel scales and rounds the accumulator
-// afterwards. The reductions (32 KB per step and SM) run at the rate the L2 accepts them, about
-// 13 bytes per clock and SM, which is what bounds this pass.
+// afterwards. At D = 128 what bounds the pass is shared-memory bandwidth: operands, dS^T and the dQ staging move
+// about 290 KB per step against 128 bytes per clock.
+//
+// DUO (the fused pass at D <= 64): two blocks per SM. The products of a step are short there and the softmax groups of
+// one block spend half their time on their own latencies, and with short sequences a block's start-up, first loads and
+// output stores weigh as much as its steps; a second block fills both. Each has half the TMEM, which leaves one
+// (T1, T2) buffer, so its steps are serial. Measured, one block per SM -> two: training step B64 H32 512 x 512 D64
+// causal fp16 (forward included) 1105 -> 945 us, B16 H16 2048 x 2048 D64 with dropout 4085 -> 3590 us; at D = 32, two
+// separate passes -> this one: B2 H16 4096 x 4096 causal bf16 455 -> 387 us.
 //
 // Per-query statistics come from a padded scratch array holding, per pair of queries, the float4
 // (-lse[m]*log2e, -lse[m+1]*log2e, -delta[m], -delta[m+1]); it is padded to a multiple of 128
@@ -69,7 +75,11 @@ struct BwdArgs {
 
 template <int D, int MODE, bool FUSED = false>
 struct BwdSmem {
-  static constexpr int STAGES = (FUSED && D == 128) ? 3 : 4;
+  // Two blocks per SM, each with half the TMEM, one (T1, T2) buffer and two ring stages.
+  static constexpr bool DUO = FUSED && D <= 64;
+  static constexpr int STAGES = DUO ? 2 : (FUSED && D == 128) ? 3 : 4;
+  static constexpr int NBUF = DUO ? 1 : 2;                     // (T1, T2) buffers
+  static constexpr int TMEM_COLS = DUO ? 256 : 512;
   static constexpr int N_A = MODE == MODE_TOTAL ? 1 : 2;       // resident tiles
   static constexpr int N_B = MODE == MODE_TOTAL ? 1 : 2;       // streamed tiles per stage
   static constexpr int A_BYTES = N_A * TileCfg<D>::TILE_BYTES; // 128 x D each
@@ -82,21 +92,29 @@ struct BwdSmem {
   static constexpr int DQ_STAGE_OFFSET = DS_OFFSET + (FUSED ? DS_TILE_BYTES : 0);
   static constexpr int BAR_OFFSET = DQ_STAGE_OFFSET + (FUSED ? 2 * DQ_STAGE_BYTES : 0);
   static constexpr int TOTAL = BAR_OFFSET + 512 + 1024;
-  static constexpr int THREADS = FUSED ? 448 : 320;
+  // Softmax groups of four warps; each owns half of the 64 columns of every step. (One block per SM with four groups of
+  // 16 columns measured 2 to 3 % slower at D = 128 and no faster at D = 64.)
+  static constexpr int GROUPS = 2;
+  // FUSED: the warps that read dQ^T back, one per 32 of its D live lanes (a warp w reaches lanes 32 (w % 4) and up).
+  static constexpr int DQ_WARPS = !FUSED ? 0 : D / 32;
+  static constexpr int MMA_WARP = DUO ? 4 * GROUPS + DQ_WARPS : 4 * GROUPS, TMA_WARP = MMA_WARP + 1;
+  static constexpr int DQ_WARP = DUO ? 4 * GROUPS : 4 * GROUPS + 2;
+  static constexpr int THREADS = 32 * (4 * GROUPS + 2 + DQ_WARPS);
 };
 
 template <int D, bool BF16, bool DROPOUT, int MODE, bool FUSED = false>
-__global__ void __launch_bounds__((BwdSmem<D, MODE, FUSED>::THREADS), 1)
+__global__ void __launch_bounds__((BwdSmem<D, MODE, FUSED>::THREADS), (BwdSmem<D, MODE, FUSED>::DUO ? 2 : 1))
 bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUtensorMap tmA2,
            const __grid_constant__ CUtensorMap tmB1, const __grid_constant__ CUtensorMap tmB2,
            const __grid_constant__ CUtensorMap tmO1, const __grid_constant__ CUtensorMap tmO2,
            const BwdArgs args) {
   using Cfg = TileCfg<D>;
   using Sm = BwdSmem<D, MODE, FUSED>;
-  static_assert(!FUSED || (MODE == MODE_KV && (D == 128 || D == 64)),
-                "the fused dQ pass exists for MODE_KV, D = 128 and 64");
+  static_assert(!FUSED || (MODE == MODE_KV && D >= 32), "the fused dQ pass exists for MODE_KV, D >= 32");
   constexpr int STAGES = Sm::STAGES;
+  constexpr int GROUPS = Sm::GROUPS;
   constexpr int STEP = 64;                                  // columns per step
+  constexpr int HALF = STEP / GROUPS;                       // ... and per softmax group
   constexpr int CHUNK_BYTES_B = STEP * Cfg::ROW_BYTES;      // one [64 x CHUNK] box
   constexpr uint64_t MN_DESC_B = make_smem_desc_hi(CHUNK_BYTES_B, 8 * Cfg::ROW_BYTES, Cfg::UMMA_SWZ);
   constexpr int N_ACC = MODE == MODE_KV ? 2 : (MODE == MODE_Q ? 1 : 0);
@@ -104,17 +122,15 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
   // When TMEM has room, the resident tiles are copied into it once (tcgen05.cp) and the T products
   // read their A operand from there: with 64-column steps those products are otherwise limited by
   // shared-memory bandwidth (both operands streamed from shared memory for every step).
-  constexpr uint32_t A_BASE = BUF_BASE + 256;               // TMEM column of the resident copies
-  constexpr bool A_IN_TMEM = A_BASE + Sm::N_A * (D / 2) <= 512;
-  // FUSED: where dQ^T (64 fp32 columns) lives. D = 128 has no free columns, so it takes the step's
-  // T2 columns once dP^T has been consumed; D = 64 has 64 columns left after the resident copies.
-  constexpr bool DQ_ALIASED = D == 128;
-  constexpr uint32_t DQ_COL_FIXED = A_BASE + Sm::N_A * (D / 2);
-  static_assert(!FUSED || DQ_ALIASED || DQ_COL_FIXED + 64 <= 512, "no TMEM columns for dQ^T");
-  auto dq_col = [](int buf) -> uint32_t { return DQ_ALIASED ? BUF_BASE + buf * 128 + 64 : DQ_COL_FIXED; };
-  // (single fixed buffer: one barrier pair, phase = step parity; aliased: one pair per T buffer)
-  auto dq_slot = [](int i) -> int { return DQ_ALIASED ? (i & 1) : 0; };
-  auto dq_phase = [](int i) -> uint32_t { return DQ_ALIASED ? ((i >> 1) & 1) : (i & 1); };
+  constexpr bool DUO = Sm::DUO;
+  constexpr int NBUF = Sm::NBUF;
+  constexpr uint32_t A_BASE = BUF_BASE + NBUF * 128;        // TMEM column of the resident copies
+  constexpr bool A_IN_TMEM = A_BASE + Sm::N_A * (D / 2) <= Sm::TMEM_COLS;
+  // FUSED: dQ^T (64 fp32 columns) takes the step's T2 columns once dP^T has been consumed.
+  auto dq_col = [](int buf) -> uint32_t { return BUF_BASE + buf * 128 + 64; };
+  // (T1, T2) buffer of step i and the phase of its barriers
+  auto buf_of = [](int i) -> int { return NBUF == 2 ? (i & 1) : 0; };
+  auto buf_phase = [](int i) -> uint32_t { return NBUF == 2 ? ((i >> 1) & 1) : (i & 1); };
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -125,7 +141,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
   uint64_t* a_full = bars;                 // [1]
   uint64_t* b_full = bars + 1;             // [STAGES]
   uint64_t* b_empty = b_full + STAGES;     // [STAGES]
-  uint64_t* t_full = b_empty + STAGES;     // [2]
+  uint64_t* t_full = b_empty + STAGES;     // [2] T1 and T2 of buffer 0 / 1 (DUO: T1 / T2 of the one buffer)
   uint64_t* p_ready = t_full + 2;          // [2]
   uint64_t* acc_full = p_ready + 2;        // [1]
   uint64_t* dq_ready = acc_full + 1;       // [2] FUSED: dQ^T of the step is complete in TMEM
@@ -192,17 +208,17 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&t_full[i], 1);
-      mbar_init(&p_ready[i], 256);
+      mbar_init(&p_ready[i], 128 * GROUPS);
       mbar_init(&dq_ready[i], 1);
-      mbar_init(&dq_drained[i], 128);
+      mbar_init(&dq_drained[i], FUSED ? 32 * Sm::DQ_WARPS : 1);
     }
     mbar_init(acc_full, 1);
-    mbar_init(epi_sync, 8);
+    mbar_init(epi_sync, 4 * GROUPS);
     *abort_flag = 0;
     fence_barrier_init();
   }
-  if (warp == 8) {
-    tmem_alloc(tmem_slot, 512);
+  if (warp == Sm::MMA_WARP) {
+    tmem_alloc(tmem_slot, Sm::TMEM_COLS);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -218,7 +234,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
     return bounded_wait(bar, parity, abort_flag, args.status, WAIT_LIMIT_NS);
   };
 
-  if (warp == 9) {
+  if (warp == Sm::TMA_WARP) {
     // ------------------------------------------------------------ TMA producer
     if (lane == 0 && T > 0) {
       tma_prefetch_desc(&tmA1);
@@ -260,7 +276,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
       }
     }
     __syncwarp();
-  } else if (warp == 8) {
+  } else if (warp == Sm::MMA_WARP) {
     // ------------------------------------------------------------- MMA issuer
     // The whole warp runs this loop with warp-uniform values; one elected lane issues each
     // tcgen05 instruction (see mma_ss_w).
@@ -284,12 +300,12 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
             tmem_cp_128x256b_w(tmem_base + A_BASE + which * (D / 2) + s * 8, da + (a_offset(which, s) >> 4));
         }
       };
-      auto issue_t = [&](int buf, int st) {
+      auto issue_t = [&](int buf, int st, int first, int last) {
         const uint32_t t1 = tmem_base + BUF_BASE + buf * 128;
         const uint64_t da = smem_desc(Cfg::KMAJOR_DESC, a_addr);
         const uint64_t db = smem_desc(Cfg::KMAJOR_DESC, b_addr + st * Sm::STAGE_BYTES);
 #pragma unroll
-        for (int which = 0; which < Sm::N_A; ++which) {
+        for (int which = first; which < last; ++which) {
 #pragma unroll
           for (int s = 0; s < D / 16; ++s) {
             const uint32_t b_off = which * Sm::B_TILE_BYTES + (s / Cfg::STEPS_PER_CHUNK) * CHUNK_BYTES_B +
@@ -309,18 +325,18 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
       // acc[which] += (P or dS from TMEM) x streamed tile `tile` of stage `st`, read MN-major.
       auto issue_acc = [&](int acc, int buf, int src, int st, int tile, bool accumulate) {
         const uint32_t d = tmem_base + acc * D;
-        // Softmax group g leaves its 32 columns' P (8+8 packed columns) at T1[32g, 32g+16) and
-        // its dS at T1[32g+16, 32g+32): K-step s covers columns 16s..16s+15 of the step.
-        const uint32_t a = tmem_base + BUF_BASE + buf * 128 + src * 16;
+        // Softmax group g leaves its HALF columns' P (HALF / 2 packed columns) at T1[HALF g] and its dS
+        // behind it at T1[HALF g + HALF / 2]: K-step s covers columns 16s..16s+15 of the step.
+        const uint32_t a = tmem_base + BUF_BASE + buf * 128 + src * (HALF / 2);
         const uint64_t db = smem_desc(MN_DESC_B, b_addr + st * Sm::STAGE_BYTES + tile * Sm::B_TILE_BYTES);
 #pragma unroll
         for (int s = 0; s < STEP / 16; ++s)
-          mma_ts_w(d, a + (s >> 1) * 32 + (s & 1) * 8, db + ((s * 16 * Cfg::ROW_BYTES) >> 4), IDESC_ACC,
+          mma_ts_w(d, a + (16 * s / HALF) * HALF + (16 * s % HALF) / 2, db + ((s * 16 * Cfg::ROW_BYTES) >> 4), IDESC_ACC,
                    (accumulate || s > 0) ? 1u : 0u);
       };
       // FUSED: dQ^T (feature rows x 64 queries) = K^T dS^T. The product always has M = 128: at
-      // D = 64 the MN-major descriptor runs on from the K tile into the V tile behind it, so lanes
-      // 64..127 receive V^T dS^T, which nobody reads.
+      // D <= 64 the MN-major descriptor runs on from the K tile into what lies behind it in shared memory, so
+      // lanes D..127 receive numbers that nobody reads.
       auto issue_dq = [&](int buf) {
         constexpr uint32_t IDESC_DQ = make_idesc(BF16, 128, STEP, true, true);
         constexpr uint64_t DS_DESC = make_smem_desc_hi(Sm::DS_TILE_BYTES, 1024, SWZ_128B);
@@ -338,46 +354,42 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
       if (ok) {
         tc_fence_after();
         if constexpr (A_IN_TMEM) stage_resident();
-        issue_t(0, 0);
+        issue_t(0, 0, 0, DUO ? 1 : Sm::N_A);
         tc_commit_w(&t_full[0]);
+        if constexpr (DUO) {
+          issue_t(0, 0, 1, 2);
+          tc_commit_w(&t_full[1]);
+        }
       }
       for (int i = 0; i < T && ok; ++i) {
-        const int buf = i & 1;
+        const int buf = buf_of(i);
         const int st = i % STAGES;
-        if (i + 1 < T) {
+        if (!DUO && i + 1 < T) {
           const int st_next = (i + 1) % STAGES;
           const bool w = wait(&b_full[st_next], ((i + 1) / STAGES) & 1);
           if (!__all_sync(0xffffffffu, w)) { fail(ST_WAIT_TMA); ok = false; break; }
-          if constexpr (FUSED && DQ_ALIASED) {
+          if constexpr (FUSED) {
             // the T2 columns of the other buffer still hold dQ^T of step i - 1 until it is read back
             if (i >= 1) {
-              const bool w2 = wait(&dq_drained[dq_slot(i - 1)], dq_phase(i - 1));
+              const bool w2 = wait(&dq_drained[buf_of(i - 1)], buf_phase(i - 1));
               if (!__all_sync(0xffffffffu, w2)) { fail(ST_WAIT_SOFTMAX); ok = false; break; }
             }
           }
           tc_fence_after();
-          issue_t(buf ^ 1, st_next);
+          issue_t(buf ^ 1, st_next, 0, Sm::N_A);
           tc_commit_w(&t_full[buf ^ 1]);
         }
         {
-          const bool w = wait(&p_ready[buf], (i >> 1) & 1);
+          const bool w = wait(&p_ready[buf], buf_phase(i));
           if (!__all_sync(0xffffffffu, w)) { fail(ST_WAIT_SOFTMAX); ok = false; break; }
         }
         tc_fence_after();
         if constexpr (MODE == MODE_KV) {
           if constexpr (FUSED) {
-            if constexpr (!DQ_ALIASED) {
-              // one fixed dQ^T buffer: the previous step's must have been read back
-              if (i >= 1) {
-                const bool w2 = wait(&dq_drained[0], dq_phase(i - 1));
-                if (!__all_sync(0xffffffffu, w2)) { fail(ST_WAIT_SOFTMAX); ok = false; break; }
-                tc_fence_after();
-              }
-            }
-            // first, so that its read-back overlaps the two accumulating products and (aliased)
+            // first, so that its read-back overlaps the two accumulating products and
             // the T2 columns are free again when the next T products are issued
             issue_dq(buf);
-            tc_commit_w(&dq_ready[dq_slot(i)]);
+            tc_commit_w(&dq_ready[buf]);
           }
           issue_acc(1, buf, 0, st, 1, i > 0);  // dV += P^T  dO
           issue_acc(0, buf, 1, st, 0, i > 0);  // dK += dS^T Q
@@ -385,42 +397,63 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
           issue_acc(0, buf, 1, st, 0, i > 0);  // dQ += dS K
         }
         tc_commit_w(&b_empty[st]);
+        if constexpr (DUO) {
+          // One buffer: the next step's products follow the ones that read P and dS out of it; T2 also waits until
+          // dQ^T has been read back. The other block of the SM works meanwhile.
+          if (i + 1 < T) {
+            const int st_next = (i + 1) % STAGES;
+            const bool w = wait(&b_full[st_next], ((i + 1) / STAGES) & 1);
+            if (!__all_sync(0xffffffffu, w)) { fail(ST_WAIT_TMA); ok = false; break; }
+            tc_fence_after();
+            issue_t(0, st_next, 0, 1);
+            tc_commit_w(&t_full[0]);
+            const bool w2 = wait(&dq_drained[0], buf_phase(i));
+            if (!__all_sync(0xffffffffu, w2)) { fail(ST_WAIT_SOFTMAX); ok = false; break; }
+            tc_fence_after();
+            issue_t(0, st_next, 1, 2);
+            tc_commit_w(&t_full[1]);
+          }
+        }
       }
       if (ok) tc_commit_w(acc_full);
     }
     __syncwarp();
-  } else if (warp >= 10) {
+  } else if (warp >= Sm::DQ_WARP) {
     // ------------------------------------------------- FUSED: dQ^T read-back and global reduction
     if constexpr (FUSED) {
       const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
       const int d = (warp & 3) * 32 + lane;  // feature index = TMEM lane
       for (int i = 0; i < T; ++i) {
-        const int buf = i & 1;
+        const int buf = buf_of(i);
         const int hh = (i + i_skip) / steps_per_head;
         const int col = col_lo + (i + i_skip - hh * steps_per_head) * STEP;
         {
           // The four warps decide together whether to go on: they meet at named barriers below, so
           // one of them leaving alone would strand the others there. Each warp's own wait is bounded,
           // hence all four reach this reduction barrier.
-          const bool w = wait(&dq_ready[dq_slot(i)], dq_phase(i));
+          const bool w = wait(&dq_ready[buf], buf_phase(i));
           uint32_t all_ok;
           asm volatile(
               "{\n\t"
               ".reg .pred p, q;\n\t"
               "setp.ne.b32 p, %1, 0;\n\t"
-              "bar.red.and.pred q, 2, 128, p;\n\t"
+              "bar.red.and.pred q, 2, %2, p;\n\t"
               "selp.b32 %0, 1, 0, q;\n\t"
               "}\n"
-              : "=r"(all_ok) : "r"(static_cast<uint32_t>(w)) : "memory");
+              : "=r"(all_ok) : "r"(static_cast<uint32_t>(w)), "n"(32 * Sm::DQ_WARPS) : "memory");
           if (!all_ok) { if (!w) fail(ST_WAIT_MMA); break; }
         }
         tc_fence_after();
-        uint32_t v[STEP];
+        // (DUO: 32 columns at a time, half the registers)
+        constexpr int HELD = DUO ? 32 : STEP;
+        uint32_t v[HELD];
         tmem_ld32(tmem_base + lane_base + dq_col(buf), v);
-        tmem_ld32(tmem_base + lane_base + dq_col(buf) + 32, v + 32);
+        if constexpr (!DUO) tmem_ld32(tmem_base + lane_base + dq_col(buf) + 32, v + HELD - 32);
         tmem_wait_ld();
-        tc_fence_before();
-        mbar_arrive(&dq_drained[dq_slot(i)]);
+        if constexpr (!DUO) {
+          tc_fence_before();
+          mbar_arrive(&dq_drained[buf]);
+        }
         // Out through shared memory, 32 queries at a time: the tile is laid out like the
         // accumulator rows ([query][feature], contiguous in global memory) and one bulk
         // reduction adds it to the fp32 accumulator.
@@ -431,15 +464,21 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
         for (int half = 0; half < 2; ++half) {
           const int rows_out = min(32, n_valid - half * 32);
           // two staging tiles: this one was last read by the reduction issued two halves ago
-          if (threadIdx.x == 320) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-          asm volatile("bar.sync 2, 128;" ::: "memory");
+          if (threadIdx.x == 32 * Sm::DQ_WARP) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          asm volatile("bar.sync 2, %0;" ::"n"(32 * Sm::DQ_WARPS) : "memory");
           float* stage = stage0 + half * (Sm::DQ_STAGE_BYTES / 4);
 #pragma unroll
           for (int c = 0; c < 32; ++c)
-            if (d < D) stage[c * D + d] = __uint_as_float(v[half * 32 + c]);
+            stage[c * D + d] = __uint_as_float(v[(DUO ? 0 : half * 32) + c]);
+          if (DUO && half == 0) {
+            tmem_ld32(tmem_base + lane_base + dq_col(buf) + 32, v);
+            tmem_wait_ld();
+            tc_fence_before();
+            mbar_arrive(&dq_drained[buf]);
+          }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          asm volatile("bar.sync 2, 128;" ::: "memory");
-          if (threadIdx.x == 320 && rows_out > 0) {
+          asm volatile("bar.sync 2, %0;" ::"n"(32 * Sm::DQ_WARPS) : "memory");
+          if (threadIdx.x == 32 * Sm::DQ_WARP && rows_out > 0) {
             asm volatile(
                 "cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;"
                 ::"l"(dst + half * 32 * D), "r"(smem_u32(stage)), "r"(rows_out * D * 4)
@@ -449,7 +488,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
         }
       }
       // the staging tile must outlive the reductions that read it
-      if (threadIdx.x == 320) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+      if (threadIdx.x == 32 * Sm::DQ_WARP) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     }
   } else {
     // --------------------------------------------------------- softmax groups
@@ -476,12 +515,10 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
     const int my_d_min = MODE == MODE_Q ? max(args.d_min, row - args.M + 1) : args.d_min;
     const int my_d_max = (MODE != MODE_Q && row >= args.N) ? -BAND_INF - 2 : args.d_max;
 
-    // Both groups work on every step: group `wg` owns columns [32*wg, 32*wg + 32) of the step, which
-    // halves the latency between the T products and the accumulating products of a step.
-    constexpr int HALF = STEP / 2;
+    // Every group works on every step: group `wg` owns columns [HALF * wg, HALF * (wg + 1)) of the step.
     for (int i = 0; i < T; ++i) {
       const int st = i % STAGES;
-      const int buf = i & 1;
+      const int buf = buf_of(i);
       const int hh = (i + i_skip) / steps_per_head;
       const int col0 = col_lo + (i + i_skip - hh * steps_per_head) * STEP + wg * HALF;  // first column of this group
       const int h = h_first + hh;
@@ -522,20 +559,23 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
         }
       }
       {
-        const bool w = wait(&t_full[buf], (i >> 1) & 1);
+        const bool w = wait(&t_full[buf], buf_phase(i));
         if (!__all_sync(0xffffffffu, w)) { if (!w) fail(ST_WAIT_MMA); ok = false; break; }
       }
       tc_fence_after();
+      // DUO (fewer registers per thread, T2 later than T1): the scores of all HALF columns are turned into
+      // probabilities first and the dP columns follow PART at a time.
+      constexpr int PART = DUO ? HALF / 2 : HALF;
       uint32_t t1[HALF];
-      uint32_t t2[MODE == MODE_TOTAL ? 1 : HALF];
+      uint32_t t2[MODE == MODE_TOTAL ? 1 : PART];
       tmem_ld32(t1_addr + wg * HALF, t1);
-      if constexpr (MODE != MODE_TOTAL) tmem_ld32(t1_addr + 64 + wg * HALF, t2);
+      if constexpr (MODE != MODE_TOTAL && !DUO) tmem_ld32(t1_addr + 64 + wg * HALF, t2);
       tmem_wait_ld();
 
       // Does this step cross the causal boundary for some row of the block?
       bool diag = false;
       if (args.causal) {
-        // d = m + P_SEQ - n ranges over [d_lo_blk, d_hi_blk] on this group's 128 x 32 block
+        // d = m + P_SEQ - n ranges over [d_lo_blk, d_hi_blk] on this group's 128 x HALF block
         int d_lo_blk, d_hi_blk;
         if constexpr (MODE == MODE_Q) {
           d_lo_blk = r0 + P_SEQ - (col0 + HALF - 1);
@@ -557,6 +597,33 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
       }
       const float4* stats4 = reinterpret_cast<const float4*>(sB + st * Sm::STAGE_BYTES + Sm::N_B * Sm::B_TILE_BYTES) +
                              wg * (HALF / 2);
+      // P and dS = P * (dP - delta) of columns c and c + 1, rounded for the products that follow
+      auto round_pair = [&](float p_a, float p_b, uint32_t dp_a, uint32_t dp_b, uint64_t ndel2, int c, uint32_t& p16,
+                            uint32_t& ds16) {
+        uint64_t dp2;
+        if constexpr (DROPOUT) {
+          dp_a &= keep_mask_one(keep_bits, c);
+          dp_b &= keep_mask_one(keep_bits, c + 1);
+          dp2 = f2_fma(f2_pack(__uint_as_float(dp_a), __uint_as_float(dp_b)), f2_pack(args.drop.inv_keep, args.drop.inv_keep), ndel2);
+        } else {
+          dp2 = f2_add(f2_pack(__uint_as_float(dp_a), __uint_as_float(dp_b)), ndel2);
+        }
+        float ds_a, ds_b;
+        f2_unpack(f2_mul(f2_pack(p_a, p_b), dp2), ds_a, ds_b);
+        p16 = pack2<BF16>(p_a, p_b);
+        if constexpr (DROPOUT) p16 &= keep_mask_pair(keep_bits, c);
+        ds16 = pack2<BF16>(ds_a, ds_b);
+      };
+      // FUSED: N columns of dS^T once more, as the shared-memory B operand of dQ^T: row = key, 64 queries = 128 bytes,
+      // 16-byte chunks permuted by the 128-byte swizzle.
+      auto share_ds = [&](int first_col, auto count, const uint32_t* ds) {
+        uint8_t* ds_row = sDS + row_local * 128;
+#pragma unroll
+        for (int j = 0; j < decltype(count)::value / 8; ++j) {
+          const int chunk = (first_col / 8 + j) ^ (row_local & 7);
+          *reinterpret_cast<uint4*>(ds_row + chunk * 16) = make_uint4(ds[4 * j + 0], ds[4 * j + 1], ds[4 * j + 2], ds[4 * j + 3]);
+        }
+      };
       // The loop exists twice, with and without the per-score visibility test, chosen once per step:
       // left as a test of `diag` inside the loop it is compiled into predicated instructions that every
       // step issues, masked or not (two more operations per pair there cost the whole pass 8 %).
@@ -564,10 +631,13 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
         constexpr bool DIAG = decltype(diag_tag)::value;
 #pragma unroll
         for (int c = 0; c < HALF; c += 2) {
-          uint64_t nlse2, ndel2;
+          uint64_t nlse2, ndel2 = 0;
           if constexpr (MODE == MODE_Q) {
             nlse2 = f2_pack(row_nlse, row_nlse);
             ndel2 = f2_pack(row_ndelta, row_ndelta);
+          } else if constexpr (DUO) {
+            const float2 sv = *reinterpret_cast<const float2*>(&stats4[c >> 1]);
+            nlse2 = f2_pack(sv.x, sv.y);
           } else {
             const float4 sv = stats4[c >> 1];
             nlse2 = f2_pack(sv.x, sv.y);
@@ -594,47 +664,57 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
           }
           if constexpr (MODE == MODE_TOTAL) {
             tot_sum += p_a + p_b;
+          } else if constexpr (DUO) {
+            t1[c] = __float_as_uint(p_a);
+            t1[c + 1] = __float_as_uint(p_b);
           } else {
-            float dp_a = __uint_as_float(t2[c]);
-            float dp_b = __uint_as_float(t2[c + 1]);
-            // dS = P * (dP - delta)
-            uint64_t dp2;
-            if constexpr (DROPOUT) {
-              dp_a = __uint_as_float(t2[c] & keep_mask_one(keep_bits, c));
-              dp_b = __uint_as_float(t2[c + 1] & keep_mask_one(keep_bits, c + 1));
-              dp2 = f2_fma(f2_pack(dp_a, dp_b), f2_pack(args.drop.inv_keep, args.drop.inv_keep), ndel2);
-            } else {
-              dp2 = f2_add(f2_pack(dp_a, dp_b), ndel2);
-            }
-            float ds_a, ds_b;
-            f2_unpack(f2_mul(f2_pack(p_a, p_b), dp2), ds_a, ds_b);
-            t1[c >> 1] = pack2<BF16>(p_a, p_b);
-            if constexpr (DROPOUT) t1[c >> 1] &= keep_mask_pair(keep_bits, c);
-            t2[c >> 1] = pack2<BF16>(ds_a, ds_b);
+            uint32_t p16, ds16;
+            round_pair(p_a, p_b, t2[c], t2[c + 1], ndel2, c, p16, ds16);
+            t1[c >> 1] = p16;
+            t2[c >> 1] = ds16;
           }
         }
       };
       if (diag) recompute(std::true_type{}); else recompute(std::false_type{});
-      if constexpr (MODE != MODE_TOTAL) {
-        // Outputs go over this group's own (already loaded) T1 columns only, so the two groups
-        // never touch each other's unread inputs.
+      // Outputs go over this group's own (already loaded) T1 columns only, so the two groups
+      // never touch each other's unread inputs.
+      if constexpr (DUO) {
+        {
+          // (T2 was issued behind the previous step's dQ^T, so it also certifies that the one tile of dS^T in shared
+          // memory may be overwritten)
+          const bool w = wait(&t_full[1], buf_phase(i));
+          if (!__all_sync(0xffffffffu, w)) { if (!w) fail(ST_WAIT_MMA); ok = false; break; }
+        }
+        tc_fence_after();
+#pragma unroll
+        for (int part = 0; part < HALF; part += PART) {
+          tmem_ld16(t1_addr + 64 + wg * HALF + part, t2);
+          tmem_wait_ld();
+          uint32_t pk[PART / 2];
+#pragma unroll
+          for (int j = 0; j < PART; j += 2) {
+            const int c = part + j;
+            const float2 sv = *(reinterpret_cast<const float2*>(&stats4[c >> 1]) + 1);
+            uint32_t ds16;
+            round_pair(__uint_as_float(t1[c]), __uint_as_float(t1[c + 1]), t2[j], t2[j + 1], f2_pack(sv.x, sv.y), c, pk[j >> 1], ds16);
+            t2[j >> 1] = ds16;
+          }
+          tmem_st8(t1_addr + wg * HALF + part / 2, pk);
+          tmem_st8(t1_addr + wg * HALF + HALF / 2 + part / 2, t2);
+          share_ds(wg * HALF + part, std::integral_constant<int, PART>{}, t2);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        tmem_wait_st();
+      } else if constexpr (MODE != MODE_TOTAL) {
         if constexpr (MODE == MODE_KV) tmem_st16(t1_addr + wg * HALF, t1);
-        tmem_st16(t1_addr + wg * HALF + 16, t2);
+        tmem_st16(t1_addr + wg * HALF + HALF / 2, t2);
         if constexpr (FUSED) {
-          // dS^T once more, as the shared-memory B operand of dQ^T: row = key, 64 queries = 128
-          // bytes, 16-byte chunks permuted by the 128-byte swizzle.
-          // (one tile: the product that read the previous step's copy must have completed)
+          // (one tile of dS^T: the product that read the previous step's copy must have completed)
           if (i >= 1) {
-            const bool w = wait(&dq_ready[dq_slot(i - 1)], dq_phase(i - 1));
+            const bool w = wait(&dq_ready[buf_of(i - 1)], buf_phase(i - 1));
             if (!__all_sync(0xffffffffu, w)) { if (!w) fail(ST_WAIT_MMA); ok = false; break; }
           }
-          uint8_t* ds_row = sDS + row_local * 128;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int chunk = (wg * 4 + j) ^ (row_local & 7);
-            *reinterpret_cast<uint4*>(ds_row + chunk * 16) =
-                make_uint4(t2[4 * j + 0], t2[4 * j + 1], t2[4 * j + 2], t2[4 * j + 3]);
-          }
+          share_ds(wg * HALF, std::integral_constant<int, HALF>{}, t2);
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
         tmem_wait_st();
@@ -649,13 +729,16 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
       if (!__all_sync(0xffffffffu, w)) { if (!w) fail(ST_WAIT_MMA); ok = false; }
     }
     if constexpr (MODE == MODE_TOTAL) {
-      // The two groups hold partial sums of alternating steps: combine through shared memory.
+      // The groups hold partial sums over different columns: combine through shared memory.
       float* red = reinterpret_cast<float*>(sA);  // the resident tile is dead after acc_full
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (wg == 1) red[row_local] = tot_sum;
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (wg == 0 && ok && row < args.N)
-        args.tot[(static_cast<int64_t>(b) * args.Hq + h_first) * args.N + row] = tot_sum + red[row_local];
+      asm volatile("bar.sync 1, %0;" ::"n"(128 * GROUPS) : "memory");
+      if (wg > 0) red[(wg - 1) * 128 + row_local] = tot_sum;
+      asm volatile("bar.sync 1, %0;" ::"n"(128 * GROUPS) : "memory");
+      if (wg == 0 && ok && row < args.N) {
+#pragma unroll
+        for (int g = 1; g < GROUPS; ++g) tot_sum += red[(g - 1) * 128 + row_local];
+        args.tot[(static_cast<int64_t>(b) * args.Hq + h_first) * args.N + row] = tot_sum;
+      }
     } else if (MODE == MODE_KV && kv_split > 1) {
       // Shared key block: this block's dK and dV go to shared memory in fp32, [accumulator][column][row], over the
       // resident tiles and the ring (all their readers have completed); summed below.
@@ -664,7 +747,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
 #pragma unroll
       for (int acc = 0; acc < N_ACC; ++acc) {
 #pragma unroll
-        for (int c = wg * (D / 2); c < (wg + 1) * (D / 2); c += 8) {
+        for (int c = wg * (D / GROUPS); c < (wg + 1) * (D / GROUPS); c += 8) {
           uint32_t o[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
           if (T > 0 && ok) {
             tmem_ld8(tmem_base + lane_base + acc * D + c, o);
@@ -675,14 +758,14 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
         }
       }
     } else if (args.out_tma) {
-      // Each thread scales and rounds its half row of every accumulator into the (now dead) resident
+      // Each thread scales and rounds its part of a row of every accumulator into the (now dead) resident
       // tile of the same index, in the swizzled layout of the output tensor map; one thread then
       // stores the 128 x D tiles with TMA, which clips rows past the end of the tensor. (Storing from
       // registers, below, writes 32 rows x 16 bytes per warp instruction and takes several
       // microseconds per CTA.) Warps that gave up still come to the meeting point.
       tc_fence_after();
       const int out_head = MODE == MODE_Q ? h_first : hk;
-      constexpr int NC = D / 2;  // columns per thread and accumulator
+      constexpr int NC = D / GROUPS;  // columns per thread and accumulator
 #pragma unroll
       for (int acc = 0; acc < N_ACC; ++acc) {
         float scale = args.sm_scale;
@@ -754,7 +837,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
                            ch * Cfg::CHUNK, r0, out_head, b);
           }
           tma_store_commit();
-          tma_store_wait_all();  // shared memory must outlive the reads of the stores
+          tma_store_wait_read();  // shared memory must outlive the reads of the stores
         }
       }
     } else if (ok) {
@@ -762,7 +845,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
       const int n_rows = MODE == MODE_Q ? args.M : args.N;
       const bool valid = row < n_rows;
       const int out_head = MODE == MODE_Q ? h_first : hk;
-      // Group `wg` converts half of the columns of every accumulator.
+      // Group `wg` converts its share of the columns of every accumulator.
 #pragma unroll
       for (int acc = 0; acc < N_ACC; ++acc) {
         void* out = acc == 0 ? args.out1 : args.out2;
@@ -772,7 +855,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
         float scale = args.sm_scale;
         if (MODE == MODE_KV && acc == 1) scale = DROPOUT ? args.drop.inv_keep : 1.0f;
 #pragma unroll
-        for (int c = wg * (D / 2); c < (wg + 1) * (D / 2); c += 8) {
+        for (int c = wg * (D / GROUPS); c < (wg + 1) * (D / GROUPS); c += 8) {
           uint32_t o[8];
           __syncwarp();
           if (T > 0) {
@@ -822,8 +905,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
       cluster_sync_all();
       const int units = D / kv_split / 8;  // groups of 8 columns per accumulator
       const int r = static_cast<int>(threadIdx.x) & 127;
-      if (threadIdx.x < 256 && r0 + r < args.N) {
-        for (int u = static_cast<int>(threadIdx.x) >> 7; u < N_ACC * units; u += 2) {
+      if (threadIdx.x < 128 * GROUPS && r0 + r < args.N) {
+        for (int u = static_cast<int>(threadIdx.x) >> 7; u < N_ACC * units; u += GROUPS) {
           const int acc = u / units, c = kv_rank * (D / kv_split) + (u - acc * units) * 8;
           const uint32_t at = smem_u32(smem) + ((acc * D + c) * 128 + r) * 4;
           float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -860,12 +943,12 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
   tc_fence_before();
   __syncthreads();
   __syncwarp();
-  if (warp == 8) {
+  if (warp == Sm::MMA_WARP) {
     if (*abort_flag) {
       const unsigned long long t0 = globaltimer_ns();
       while (globaltimer_ns() - t0 < 200000ull) {}
     }
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, Sm::TMEM_COLS);
   }
 }
 

@@ -45,8 +45,8 @@ def get_fwd_config(B, H, M, N, D, causal):
 def get_bwd_config(B, H, M, N, D, causal):
     """Counterpart of the reference's backward hook (``flash.py:514-539``); see ``get_fwd_config``.
     The backward keeps 128 rows resident per CTA and streams 64 columns per step."""
-    fused = D in (64, 128)
-    return (128, 64, 3 if D == 128 else 4, 14 if fused else 10)
+    stages, warps = {128: (3, 14), 64: (2, 12), 32: (2, 11)}.get(D, (4, 10))
+    return (128, 64, stages, warps)
 
 
 def _tma_ready(x: torch.Tensor) -> torch.Tensor:
@@ -285,7 +285,7 @@ class FlashAttentionFunction(torch.autograd.Function):
                 int(ctx.causal), float(ctx.sm_scale), float(ctx.dropout_p),
                 as_u64(ctx.seed), as_u64(ctx.offset), status.data_ptr(), 0, 0, 0,
                 ctx.keep_mask.data_ptr() if ctx.keep_mask is not None else None)
-            # At D = 128 and 64 the library produces dQ inside the dK/dV pass, summing the key blocks'
+            # At D >= 32 the library produces dQ inside the dK/dV pass, summing the key blocks'
             # contributions by fp32 reductions in global memory: faster, but the summation order (and
             # so the last bit of dQ) can differ between runs. torch.use_deterministic_algorithms(True)
             # selects the two separate kernels, whose results are reproducible bit for bit.
