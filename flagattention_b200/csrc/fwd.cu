@@ -91,12 +91,27 @@ extern "C" int b200attn_fwd(const b200attn_fwd_params* p, void* stream) {
   // it measured 0 to 4 % slower, so those launches keep the 128-key pipeline.
   int band_lo = 0, band_hi = 0;
   L.split64 = p->D == 128 && fold_band(p->causal != 0, p->band, p->dist_min, p->dist_max, &band_lo, &band_hi);
+  switch (p->D) {
+    case 16: make_o_tmap<16>(p, L); break;
+    case 32: make_o_tmap<32>(p, L); break;
+    case 64: make_o_tmap<64>(p, L); break;
+    default: make_o_tmap<128>(p, L); break;
+  }
+  // D <= 64 with 16-bit output: one query tile per block, four blocks per SM (fwd_solo.cuh), where there is a mask or
+  // the sequences are short. Forward, two tiles -> one: B4 Hq32 Hkv8 4096 causal D64 bf16 430 -> 375 us, 16384 causal
+  // 732 -> 708, B64 H32 512 causal (training step) 982 -> 820; 4096 without a mask 717 -> 726, so long launches without a
+  // mask keep the pairs, whose shared K/V tiles then pay. At D = 128 (two blocks per SM) it lost everywhere (B4 Hq16
+  // 2048 causal 82 -> 93 us).
+  L.solo = p->D <= 64 && L.args.o_tma && (fold_band(p->causal != 0, p->band, p->dist_min, p->dist_max, &band_lo, &band_hi) ||
+                                          p->N <= 1024) &&
+           static_cast<int64_t>(p->B) * p->Hq * cdiv(p->M, 128) <= 2147483647ll;
+  const int kv_rows = L.split64 || L.solo ? 64 : 128;
   int rc;
   switch (p->D) {
-    case 16: rc = make_fwd_tmaps<16>(p, L); break;
-    case 32: rc = make_fwd_tmaps<32>(p, L); break;
-    case 64: rc = make_fwd_tmaps<64>(p, L); break;
-    default: rc = make_fwd_tmaps<128>(p, L, L.split64 ? 64 : 128); break;
+    case 16: rc = make_fwd_tmaps<16>(p, L, kv_rows); break;
+    case 32: rc = make_fwd_tmaps<32>(p, L, kv_rows); break;
+    case 64: rc = make_fwd_tmaps<64>(p, L, kv_rows); break;
+    default: rc = make_fwd_tmaps<128>(p, L, kv_rows); break;
   }
   if (rc) return rc;
 
@@ -129,21 +144,15 @@ extern "C" int b200attn_fwd(const b200attn_fwd_params* p, void* stream) {
     if (rc_mask) return rc_mask;
   }
   a.status = p->status;
-  a.n_zblocks = cdiv(p->M, 256);
+  a.n_zblocks = cdiv(p->M, L.solo ? 128 : 256);
   a.grid_chunk = grid_chunk(a.groups, 4ll * p->N * p->D, a.causal != 0);
   set_item_order(a, p->Hq);
-  switch (p->D) {
-    case 16: make_o_tmap<16>(p, L); break;
-    case 32: make_o_tmap<32>(p, L); break;
-    case 64: make_o_tmap<64>(p, L); break;
-    default: make_o_tmap<128>(p, L); break;
-  }
   // One CTA per SM walks the list of work items when there are more items than SMs. The list is
   // dealt out in a fixed order, which is even when the items are equally long (no mask) and close
   // to even for short masked ones; with a mask over more than 32 K/V tiles the items differ by
   // enough that one CTA per item, placed by the hardware as SMs fall free, measured 3-7 % faster.
   a.n_items = static_cast<int>(static_cast<int64_t>(p->B) * p->Hq * a.n_zblocks);  // range checked above
-  const bool chain = a.causal == 0 || cdiv(p->N, 128) <= 32;
+  const bool chain = !L.solo && (a.causal == 0 || cdiv(p->N, 128) <= 32);
   const int n_ctas = chain ? sm_count() : a.n_items;
   L.grid = dim3(static_cast<unsigned>(a.n_items < n_ctas ? a.n_items : n_ctas));
   L.bf16 = p->dtype == B200ATTN_BF16;

@@ -2,6 +2,7 @@
 // so the variants compile in parallel.
 #pragma once
 #include "fwd_kernel.cuh"
+#include "fwd_solo.cuh"
 
 namespace b200attn {
 
@@ -10,6 +11,7 @@ struct FwdLaunch {
   FwdArgs args;
   dim3 grid;
   bool bf16, dropout;
+  bool solo = false;     // D <= 64, plain mode, 16-bit output: one query tile per block (fwd_solo.cuh)
   bool split64 = false;  // D = 128, plain mode: the 64-key softmax pipeline (fwd_kernel's SPLIT64)
   cudaStream_t stream;
 };
@@ -28,8 +30,26 @@ int launch_fwd_variant(const FwdLaunch& L) {
   return launch(CHAINED, kernel, L.grid, 384, smem, L.stream, L.tmQ, L.tmK, L.tmV, L.tmO, L.args);
 }
 
+template <int D, bool BF16, bool DROPOUT>
+int launch_fwd_solo_variant(const FwdLaunch& L) {
+  auto kernel = fwd_solo_kernel<D, BF16, DROPOUT>;
+  static PerDeviceOnce attr_once;  // one per kernel variant
+  const int rc = attr_once.run([&]() -> int {
+    B200ATTN_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SoloSmem<D>::TOTAL));
+    return B200ATTN_OK;
+  });
+  if (rc) return rc;
+  return launch(CHAINED, kernel, L.grid, SoloSmem<D>::THREADS, SoloSmem<D>::TOTAL, L.stream, L.tmQ, L.tmK, L.tmV, L.tmO, L.args);
+}
+
 template <int D>
 int launch_fwd_d(const FwdLaunch& L) {
+  if constexpr (D <= 64) {
+    if (L.solo) {
+      if (L.bf16) return L.dropout ? launch_fwd_solo_variant<D, true, true>(L) : launch_fwd_solo_variant<D, true, false>(L);
+      return L.dropout ? launch_fwd_solo_variant<D, false, true>(L) : launch_fwd_solo_variant<D, false, false>(L);
+    }
+  }
   if constexpr (D == 128) {
     if (L.split64) {
       if (L.bf16) return L.dropout ? launch_fwd_variant<D, true, true, true>(L) : launch_fwd_variant<D, true, false, true>(L);

@@ -38,6 +38,8 @@ def get_fwd_config(B, H, M, N, D, causal):
     documents its hook as replaceable at run time (``examples/use_cutom_config_func.py:18-23`` assigns
     ``flag_attn.flash.get_fwd_config``). Here tile shapes are template parameters of the CUDA kernels,
     so the function reports them and assigning another one is accepted and has no effect."""
+    if D <= 64 and (causal or N <= 1024):
+        return (128, 64, 2 if D == 64 else 4, 8)   # one 128-row query tile per CTA, 64-key steps, 256 threads
     stages = 2 if D == 128 else (3 if D == 64 else 4)
     return (256, 128, stages, 12)   # two 128-row query tiles per CTA, 128-key K/V tiles, 384 threads
 
