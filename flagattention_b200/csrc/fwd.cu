@@ -415,6 +415,8 @@ static int run_splitkv(const b200attn_splitkv_params* p, const PagedKV* paged, v
     a.bt_stride = paged->bt_stride;
     a.context_lens = paged->context_lens;
     a.block_shift = paged->block_shift;
+    const int64_t entries = static_cast<int64_t>(p->B) * cta_splits;
+    a.sort_entries = packed && entries <= 384 ? static_cast<int>(entries) : 0;  // (one thread each)
   }
   a.ring_stages = p->D == 128 ? FwdSmem<128>::DUAL_STAGES
                   : p->D == 64 ? FwdSmem<64>::DUAL_STAGES

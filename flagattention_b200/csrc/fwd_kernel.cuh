@@ -76,6 +76,10 @@ struct FwdArgs {
   int64_t bt_stride;
   const int32_t* context_lens;
   int block_shift;
+  int sort_entries;                 // > 0 (paged, packed): the (sequence, split) entries of the launch, at most one per
+                                    // thread; they are taken longest first. Sequences of a batch differ in length, and in
+                                    // their given order the last blocks run alone: 32 sequences of 1024 to 4096 keys,
+                                    // Hq64 Hkv8 D128: 92.5 -> 78 us.
   int B, Hq, Hkv, M, N, groups;
   int causal, o_fp32;               // causal: some band limit below is finite (enables the masking code)
   // Visibility band: query m sees key n iff d_min <= m + (N - M) - n < d_max. Plain causal masking is
@@ -178,6 +182,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
   uint64_t* pv_done = q_empty + 2;          // [2] SPLIT64: every P V issued so far for the tile has completed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* my_entry = reinterpret_cast<volatile int*>(tmem_slot + 2);  // sort_entries: this block's entry
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -199,9 +204,13 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     const int z_row = args.div_splits.div(bc.z);
     it.split = bc.z - z_row * args.num_splits;
     const int m_blk = args.div_splits.div(args.n_zblocks) - 1 - z_row;  // longest first
-    const int j_split = it.split * args.tiles_per_split;  // first K/V tile of this item's split
     it.b = args.div_heads.div(bc.bh);
-    const int head = bc.bh - it.b * grid_heads;
+    const int head = args.sort_entries > 0 ? id % grid_heads : bc.bh - it.b * grid_heads;
+    if (args.sort_entries > 0) {
+      it.b = *my_entry / args.num_splits;
+      it.split = *my_entry - it.b * args.num_splits;
+    }
+    const int j_split = it.split * args.tiles_per_split;  // first K/V tile of this item's split
     it.hk = packed ? head : args.div_groups.div(head);
     it.h = packed ? it.hk * args.groups : head;   // first (or only) query head
     it.m0 = m_blk * 2 * BLOCK;
@@ -273,6 +282,28 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
   const uint32_t tmem_base = *tmem_slot;
   pdl_trigger();
   pdl_wait();
+  if (args.sort_entries > 0) {
+    // Blocks id, id + 1, ... take the heads of the longest entry, then of the next: thread t ranks entry t.
+    int* tiles = reinterpret_cast<int*>(sQ);  // (no load has been issued yet)
+    const int e = static_cast<int>(threadIdx.x), n = args.sort_entries;
+    int mine = 0;
+    if (e < n) {
+      const int seq = e / args.num_splits, first = (e - seq * args.num_splits) * args.tiles_per_split;
+      mine = max(0, min(cdiv(args.context_lens[seq], BLOCK) - first, args.tiles_per_split));
+      tiles[e] = mine;
+    }
+    __syncthreads();
+    if (e < n) {
+      int rank = 0;
+      for (int j = 0; j < n; ++j) {
+        const int other = tiles[j];
+        rank += (other > mine || (other == mine && j < e)) ? 1 : 0;
+      }
+      if (rank == static_cast<int>(blockIdx.x) / grid_heads) *my_entry = e;
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the Q tile is loaded over `tiles`
+    __syncthreads();
+  }
 
   auto fail = [&](int32_t code) {
     report_status(args.status, code);
