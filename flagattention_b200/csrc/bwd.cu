@@ -174,7 +174,7 @@ static int run_bwd(const b200attn_bwd_params* p, float2* stats, cudaStream_t str
                      encode_tmap_4d(&kv.tmO2, p->dv, 2, p->B, p->Hkv, p->N, D, TileCfg<D>::CHUNK, 128,
                                     TileCfg<D>::TMA_SWZ, "dv") == B200ATTN_OK) ? 1 : 0;
   kv.args.n_zblocks = cdiv(p->N, 128);
-  kv.args.grid_chunk = grid_chunk(1, 4ll * a.groups * p->M * D, a.causal != 0);
+  kv.args.grid_chunk = grid_chunk(1, 4ll * a.groups * p->M * D, a.causal != 0, static_cast<int64_t>(p->B) * p->Hkv);
   kv.args.kv_split = bwd_kv_split(kv.args, D);
   kv.grid = dim3(static_cast<unsigned>(static_cast<int64_t>(p->B) * p->Hkv * kv.args.n_zblocks * kv.args.kv_split));
   kv.bf16 = p->dtype == B200ATTN_BF16;
@@ -190,7 +190,7 @@ static int run_bwd(const b200attn_bwd_params* p, float2* stats, cudaStream_t str
   qq.args.out_tma = encode_tmap_4d(&qq.tmO1, p->dq, 2, p->B, p->Hq, p->M, D, TileCfg<D>::CHUNK, 128,
                                    TileCfg<D>::TMA_SWZ, "dq") == B200ATTN_OK ? 1 : 0;
   qq.args.n_zblocks = cdiv(p->M, 128);
-  qq.args.grid_chunk = grid_chunk(a.groups, 4ll * p->N * D, a.causal != 0);
+  qq.args.grid_chunk = grid_chunk(a.groups, 4ll * p->N * D, a.causal != 0, static_cast<int64_t>(p->B) * p->Hkv);
   qq.grid = dim3(static_cast<unsigned>(static_cast<int64_t>(p->B) * p->Hq * qq.args.n_zblocks));
   qq.bf16 = kv.bf16;
   qq.dropout = kv.dropout;
@@ -252,7 +252,7 @@ static int run_total(const b200attn_total_params* p, float2* stats, cudaStream_t
   a.status = p->status;
   L.args = a;
   L.args.n_zblocks = cdiv(p->N, 128);
-  L.args.grid_chunk = grid_chunk(1, 2ll * p->M * D, a.causal != 0);
+  L.args.grid_chunk = grid_chunk(1, 2ll * p->M * D, a.causal != 0, static_cast<int64_t>(p->B) * p->Hq);
   L.grid = dim3(static_cast<unsigned>(static_cast<int64_t>(p->B) * p->Hq * L.args.n_zblocks));
   L.bf16 = p->dtype == B200ATTN_BF16;
   L.dropout = false;

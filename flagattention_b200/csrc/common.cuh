@@ -362,13 +362,17 @@ struct BlockOrder {
   }
 };
 // Number of (batch, head) pairs per chunk: all query heads of as many KV heads as fit `budget`
-// bytes of streamed operand per KV head (`bytes_per_kv_head`), at least one KV head.
-__host__ inline int grid_chunk(int groups, int64_t bytes_per_kv_head, bool causal) {
+// bytes of streamed operand per KV head (`bytes_per_kv_head`), at least one KV head, and the chunks about equally large:
+// a small last chunk starts its long blocks when nothing else is left to run beside them. (`kv_heads` in all, with
+// batch. 32 of them, 22 to a budget: chunks of 22 and 10 -> 16 and 16, training step B4 Hq32 Hkv8 4096 causal D64
+// 1740 -> 1530 us; B4 Hq32 Hkv8 2048 D128 665 -> 608.)
+__host__ inline int grid_chunk(int groups, int64_t bytes_per_kv_head, bool causal, int64_t kv_heads) {
   if (!causal) return groups;
   const int64_t budget = 96ll << 20;
   int64_t n = budget / (bytes_per_kv_head > 0 ? bytes_per_kv_head : 1);
   if (n < 1) n = 1;
   if (n > 4096) n = 4096;
+  n = cdiv(kv_heads, cdiv(kv_heads, n));
   return static_cast<int>(n) * groups;
 }
 

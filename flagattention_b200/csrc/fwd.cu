@@ -145,7 +145,7 @@ extern "C" int b200attn_fwd(const b200attn_fwd_params* p, void* stream) {
   }
   a.status = p->status;
   a.n_zblocks = cdiv(p->M, L.solo ? 128 : 256);
-  a.grid_chunk = grid_chunk(a.groups, 4ll * p->N * p->D, a.causal != 0);
+  a.grid_chunk = grid_chunk(a.groups, 4ll * p->N * p->D, a.causal != 0, static_cast<int64_t>(p->B) * p->Hkv);
   set_item_order(a, p->Hq);
   // One CTA per SM walks the list of work items when there are more items than SMs. The list is
   // dealt out in a fixed order, which is even when the items are equally long (no mask) and close
@@ -430,7 +430,7 @@ static int run_splitkv(const b200attn_splitkv_params* p, const PagedKV* paged, v
   a.drop = make_dropout_ctx(0.f, 0, 0);
   a.status = p->status;
   a.n_zblocks = cdiv(p->M, 256) * cta_splits;
-  a.grid_chunk = packed ? 1 : grid_chunk(a.groups, 4ll * p->N * p->D, a.causal != 0);
+  a.grid_chunk = packed ? 1 : grid_chunk(a.groups, 4ll * p->N * p->D, a.causal != 0, static_cast<int64_t>(p->B) * p->Hkv);
   set_item_order(a, packed ? p->Hkv : p->Hq);
   a.o_tma = 0;  // fp32 partial outputs are stored from registers
   const int64_t n_items = static_cast<int64_t>(p->B) * (packed ? p->Hkv : p->Hq) * a.n_zblocks;
