@@ -415,8 +415,9 @@ static int run_splitkv(const b200attn_splitkv_params* p, const PagedKV* paged, v
     a.bt_stride = paged->bt_stride;
     a.context_lens = paged->context_lens;
     a.block_shift = paged->block_shift;
+    // (one thread each; with at most one block per SM the order is of no use and ranking costs 1.5 us)
     const int64_t entries = static_cast<int64_t>(p->B) * cta_splits;
-    a.sort_entries = packed && entries <= 384 ? static_cast<int>(entries) : 0;  // (one thread each)
+    a.sort_entries = packed && entries <= 384 && entries * p->Hkv > sm_count() ? static_cast<int>(entries) : 0;
   }
   a.ring_stages = p->D == 128 ? FwdSmem<128>::DUAL_STAGES
                   : p->D == 64 ? FwdSmem<64>::DUAL_STAGES
