@@ -106,6 +106,7 @@ class SelftestParams(Structure):
 # name -> (restype, argtypes); every symbol include/b200attn.h declares.
 SYMBOLS = {
     "b200attn_fwd": (c_int32, [POINTER(FwdParams), c_void_p]),
+    "b200attn_fwd_merge": (c_int32, [POINTER(FwdParams), c_void_p, c_void_p, c_void_p]),
     "b200attn_total_workspace_bytes": (c_size_t, [c_int32] * 3),
     "b200attn_total_attention": (c_int32, [POINTER(TotalParams), c_void_p]),
     "b200attn_total_attention_static": (c_int32, [POINTER(TotalParams), c_void_p]),

@@ -38,7 +38,8 @@ static void make_o_tmap(const b200attn_fwd_params* p, FwdLaunch& L) {
 
 }  // namespace b200attn
 
-extern "C" int b200attn_fwd(const b200attn_fwd_params* p, void* stream) {
+// merge_o, merge_lse: see b200attn_fwd_merge(); null for a plain forward.
+static int run_fwd(const b200attn_fwd_params* p, const float* merge_o, const float* merge_lse, void* stream) {
   using namespace b200attn;
   if (p == nullptr) {
     set_error("fwd: null params");
@@ -90,7 +91,7 @@ extern "C" int b200attn_fwd(const b200attn_fwd_params* p, void* stream) {
   // 128-key pipeline: +3 % to +6 % on causal sequences of 2k to 32k keys, +23 % at 512; without a mask
   // it measured 0 to 4 % slower, so those launches keep the 128-key pipeline.
   int band_lo = 0, band_hi = 0;
-  L.split64 = p->D == 128 && fold_band(p->causal != 0, p->band, p->dist_min, p->dist_max, &band_lo, &band_hi);
+  L.split64 = p->D == 128 && (merge_o != nullptr || fold_band(p->causal != 0, p->band, p->dist_min, p->dist_max, &band_lo, &band_hi));
   switch (p->D) {
     case 16: make_o_tmap<16>(p, L); break;
     case 32: make_o_tmap<32>(p, L); break;
@@ -102,7 +103,7 @@ extern "C" int b200attn_fwd(const b200attn_fwd_params* p, void* stream) {
   // 732 -> 708, B64 H32 512 causal (training step) 982 -> 820; 4096 without a mask 717 -> 726, so long launches without a
   // mask keep the pairs, whose shared K/V tiles then pay. At D = 128 (two blocks per SM) it lost everywhere (B4 Hq16
   // 2048 causal 82 -> 93 us).
-  L.solo = p->D <= 64 && L.args.o_tma && (fold_band(p->causal != 0, p->band, p->dist_min, p->dist_max, &band_lo, &band_hi) ||
+  L.solo = p->D <= 64 && L.args.o_tma && merge_o == nullptr && (fold_band(p->causal != 0, p->band, p->dist_min, p->dist_max, &band_lo, &band_hi) ||
                                           p->N <= 1024) &&
            static_cast<int64_t>(p->B) * p->Hq * cdiv(p->M, 128) <= 2147483647ll;
   const int kv_rows = L.split64 || L.solo ? 64 : 128;
@@ -144,6 +145,12 @@ extern "C" int b200attn_fwd(const b200attn_fwd_params* p, void* stream) {
     if (rc_mask) return rc_mask;
   }
   a.status = p->status;
+  a.merge_o = merge_o;
+  a.merge_lse = merge_lse;
+  if (merge_o != nullptr && !a.o_tma) {
+    set_error("fwd_merge: o cannot be described by a tensor map");
+    return B200ATTN_EUNSUPPORTED;
+  }
   a.n_zblocks = cdiv(p->M, L.solo ? 128 : 256);
   a.grid_chunk = grid_chunk(a.groups, 4ll * p->N * p->D, a.causal != 0, static_cast<int64_t>(p->B) * p->Hkv);
   set_item_order(a, p->Hq);
@@ -164,6 +171,21 @@ extern "C" int b200attn_fwd(const b200attn_fwd_params* p, void* stream) {
     case 64: return launch_fwd_d64(L);
     default: return launch_fwd_d128(L);
   }
+}
+
+extern "C" int b200attn_fwd(const b200attn_fwd_params* p, void* stream) { return run_fwd(p, nullptr, nullptr, stream); }
+
+extern "C" int b200attn_fwd_merge(const b200attn_fwd_params* p, const float* o_part, const float* lse_part, void* stream) {
+  using namespace b200attn;
+  if (p == nullptr || o_part == nullptr || lse_part == nullptr || reinterpret_cast<uintptr_t>(o_part) % 16 != 0) {
+    set_error("fwd_merge: null argument or o_part not 16-byte aligned");
+    return B200ATTN_EINVAL;
+  }
+  if (!p->band || p->dropout_p != 0.f || p->o_dtype != p->dtype) {
+    set_error("fwd_merge: needs a band, no dropout and a 16-bit output");
+    return B200ATTN_EINVAL;
+  }
+  return run_fwd(p, o_part, lse_part, stream);
 }
 
 // ------------------------------------------------------------------ split-KV

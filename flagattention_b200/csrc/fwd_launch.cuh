@@ -16,9 +16,9 @@ struct FwdLaunch {
   cudaStream_t stream;
 };
 
-template <int D, bool BF16, bool DROPOUT, bool SPLIT64 = false>
+template <int D, bool BF16, bool DROPOUT, bool SPLIT64 = false, bool MERGE = false>
 int launch_fwd_variant(const FwdLaunch& L) {
-  auto kernel = fwd_kernel<D, BF16, DROPOUT, SPLIT64>;
+  auto kernel = fwd_kernel<D, BF16, DROPOUT, SPLIT64, MERGE>;
   constexpr int smem_max = FwdSmem<D>::TOTAL > FwdSmem<D>::DUAL_TOTAL ? FwdSmem<D>::TOTAL : FwdSmem<D>::DUAL_TOTAL;
   const int smem = L.args.dual_stream ? FwdSmem<D>::DUAL_TOTAL : FwdSmem<D>::TOTAL;
   static PerDeviceOnce attr_once;  // one per kernel variant
@@ -44,6 +44,9 @@ int launch_fwd_solo_variant(const FwdLaunch& L) {
 
 template <int D>
 int launch_fwd_d(const FwdLaunch& L) {
+  if (L.args.merge_o != nullptr) {  // (no dropout; D = 128 always with a band here)
+    return L.bf16 ? launch_fwd_variant<D, true, false, D == 128, true>(L) : launch_fwd_variant<D, false, false, D == 128, true>(L);
+  }
   if constexpr (D <= 64) {
     if (L.solo) {
       if (L.bf16) return L.dropout ? launch_fwd_solo_variant<D, true, true>(L) : launch_fwd_solo_variant<D, true, false>(L);

@@ -4,10 +4,10 @@ this library's kernels.
 ``S[m, n] = q2[m]·k2[n]`` where the distance ``m + (N - M) - n`` is at least ``dist_threshold`` and
 ``q1[m]·k1[n]`` elsewhere; one softmax over the whole row; ``o = P v``. The two regions are disjoint
 bands of the distance, so the row's softmax is the normaliser-weighted merge of two band-limited
-attentions: the forward runs the forward kernel once per (q, k) pair with the band mask of its region
-(``b200attn_fwd`` with ``band``), writing fp32 partial outputs and log-normalisers, and merges them
-(``b200attn_merge_partial_store``, the algebra of the split-KV combine, rounding straight into the
-output). The backward runs the backward
+attentions: the forward runs the forward kernel once per (q, k) pair with the band mask of its region,
+the near region into an fp32 partial output and log-normaliser (``b200attn_fwd`` with ``band``), the far
+region combining its rows with them in its epilogue (``b200attn_fwd_merge``, the algebra of the split-KV
+combine, rounding straight into the output). The backward runs the backward
 kernels once per pair with the same bands, both on the merged log-normaliser and on ``delta`` of the
 merged output; each call yields its pair's dQ and dK, and the two dV contributions are added.
 """
@@ -54,21 +54,22 @@ class PiecewiseAttentionFunction(torch.autograd.Function):
         with torch.cuda.device(device):
             stream = _lib.current_stream_ptr(device)
             status = _status_word(device)
-            parts = []
-            for (q, k), (dmin, dmax) in zip(((q1, k1), (q2, k2)), _bands(w, bool(causal))):
-                o_part = torch.empty((B, H, M, D), dtype=torch.float32, device=device)
-                l_part = torch.empty((B, H, M), dtype=torch.float32, device=device)
-                fp = _lib.FwdParams(
-                    _lib.tensor4(q), _lib.tensor4(k), _lib.tensor4(v), _lib.tensor4(o_part), l_part.data_ptr(),
-                    B, H, H, M, N, D, dt, _lib.dtype_code(torch.float32), int(bool(causal)), float(sm_scale),
-                    0.0, 0, 0, status.data_ptr(), 1, dmin, dmax)
-                _lib.check(lib.b200attn_fwd(fp, stream), "b200attn_fwd")
-                parts.append((o_part, l_part))
-            (o_acc, L), (o_far, l_far) = parts
+            near, far = _bands(w, bool(causal))
+            # The near region's result stays in fp32; the far region's forward combines its own rows with it.
+            o_near = torch.empty((B, H, M, D), dtype=torch.float32, device=device)
+            l_near = torch.empty((B, H, M), dtype=torch.float32, device=device)
             o = torch.empty_like(q1)
-            _lib.check(lib.b200attn_merge_partial_store(o_acc.data_ptr(), L.data_ptr(), o_far.data_ptr(),
-                                                        l_far.data_ptr(), B, H, M, D, _lib.tensor4(o), dt, stream),
-                       "b200attn_merge_partial_store")
+            L = torch.empty((B, H, M), dtype=torch.float32, device=device)
+            fp = _lib.FwdParams(
+                _lib.tensor4(q1), _lib.tensor4(k1), _lib.tensor4(v), _lib.tensor4(o_near), l_near.data_ptr(),
+                B, H, H, M, N, D, dt, _lib.dtype_code(torch.float32), int(bool(causal)), float(sm_scale),
+                0.0, 0, 0, status.data_ptr(), 1, *near)
+            _lib.check(lib.b200attn_fwd(fp, stream), "b200attn_fwd")
+            fp = _lib.FwdParams(
+                _lib.tensor4(q2), _lib.tensor4(k2), _lib.tensor4(v), _lib.tensor4(o), L.data_ptr(),
+                B, H, H, M, N, D, dt, dt, int(bool(causal)), float(sm_scale),
+                0.0, 0, 0, status.data_ptr(), 1, *far)
+            _lib.check(lib.b200attn_fwd_merge(fp, o_near.data_ptr(), l_near.data_ptr(), stream), "b200attn_fwd_merge")
         ctx.save_for_backward(q1, k1, q2, k2, v, o, L)
         ctx.sm_scale = sm_scale
         ctx.causal = bool(causal)

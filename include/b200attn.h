@@ -74,6 +74,11 @@ size_t b200attn_keep_mask_bytes(int32_t B, int32_t Hq, int32_t M, int32_t N);
 
 int b200attn_fwd(const b200attn_fwd_params* p, void* stream);
 
+/* The same for a band (p->band, no dropout, 16-bit o), combined with a partial result over other keys before it is
+ * rounded: o_part [B,Hq,M,D] and lse_part [B,Hq,M], contiguous fp32, as a forward with o_dtype B200ATTN_F32 writes them.
+ * p->o and p->lse receive the joint result (softmax over the union of the two key sets). */
+int b200attn_fwd_merge(const b200attn_fwd_params* p, const float* o_part, const float* lse_part, void* stream);
+
 /* Total attention: replaces `_total_attention_kernel` (total.py:64-156, launched
  * flash.py:147-159). tot[b,h,n] = sum_m exp(s[m,n]*sm_scale - lse[m]) over visible m.
  * `workspace` is caller-allocated scratch of b200attn_total_workspace_bytes(B, Hq, M) bytes,
