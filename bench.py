@@ -208,9 +208,9 @@ def run_step(cfg, q, k, v, do):
 
 
 def kernels_per_step(cfg) -> int:
-    # forward: 1 kernel; backward: delta, statistics, then either the dK/dV kernel and the dQ kernel
-    # or (D = 128 and 64) the fused dK/dV/dQ kernel and the dQ conversion.
-    return 1 + (4 if cfg["mode"] == "fwd+bwd" else 0)
+    # forward: 1 kernel, and the one that draws the dropout decisions; backward: preprocess, the fused dK/dV/dQ kernel
+    # (D >= 32; else the dK/dV kernel) and the dQ conversion (else the dQ kernel).
+    return 1 + (cfg["dropout_p"] > 0) + (3 if cfg["mode"] == "fwd+bwd" else 0)
 
 
 def time_kernels(cfg, inputs, iters=20, n_sets=2):
@@ -227,7 +227,7 @@ def time_kernels(cfg, inputs, iters=20, n_sets=2):
     status = torch.zeros(1, dtype=torch.int32, device=dev)
     sm_scale = 1.0 / math.sqrt(D)
     bwd = cfg["mode"] == "fwd+bwd"
-    fused = D in (64, 128)
+    fused = D >= 32
     sets = []
     for s in range(n_sets):
         q, k, v, do = (q0, k0, v0, do0) if s == 0 else (t.clone() for t in (q0, k0, v0, do0))
