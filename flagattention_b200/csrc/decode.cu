@@ -234,6 +234,8 @@ decode_partial_kernel(const DecodeArgs a) {
   // Merge the warps through shared memory.
   __shared__ float sm_m[DEC_WARPS][R], sm_l[DEC_WARPS][R];
   __shared__ float sm_acc[DEC_WARPS][R][D];
+  __shared__ float sm_part[R][D], sm_part_lse[R];  // this split's result, for the block that merges the cluster
+  const bool merged = a.final_o != nullptr && a.num_splits > 1;
   if (group == 0) {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -263,7 +265,10 @@ decode_partial_kernel(const DecodeArgs a) {
     const int g = r / a.M, m = r % a.M;
     const int64_t h = hk * a.groups + g;
     const float lse = l_tot > 0.f ? m_new * 0.6931471805599453f + logf(l_tot) : -INFINITY;
-    if (a.final_o != nullptr) {
+    if (merged) {
+      sm_part[r][d] = o;
+      if (d == 0) sm_part_lse[r] = lse;
+    } else if (a.final_o != nullptr) {
       uint16_t* dst = a.final_o + b * a.o_sb + h * a.o_sh + static_cast<int64_t>(m) * a.o_sm + d;
       if constexpr (BF16) {
         const __nv_bfloat16 v = __float2bfloat16_rn(o);
@@ -279,11 +284,51 @@ decode_partial_kernel(const DecodeArgs a) {
       if (d == 0) a.part_lse[row] = lse;
     }
   }
+  if (merged) {
+    // The algebra of splitkv_combine_kernel (fwd.cu) over the cluster's shared memory; block 0 writes.
+    __syncwarp();
+    cluster_sync_all();
+    if (split == 0) {
+      for (int idx = threadIdx.x; idx < rows * D; idx += DEC_THREADS) {
+        const int r = idx / D, d = idx % D;
+        const uint32_t at = smem_u32(&sm_part[r][d]), at_lse = smem_u32(&sm_part_lse[r]);
+        float l[DECODE_MAX_CLUSTER], x[DECODE_MAX_CLUSTER], mx = -INFINITY;
+#pragma unroll
+        for (int s = 0; s < DECODE_MAX_CLUSTER; ++s) {
+          l[s] = s < a.num_splits ? cluster_load(cluster_map(at_lse, s)) : -INFINITY;
+          x[s] = s < a.num_splits ? cluster_load(cluster_map(at, s)) : 0.f;
+          mx = fmaxf(mx, l[s]);
+        }
+        float denom = 0.f, acc = 0.f;
+#pragma unroll
+        for (int s = 0; s < DECODE_MAX_CLUSTER; ++s) {
+          const float w = mx == -INFINITY ? 0.f : expf(l[s] - mx);
+          denom += w;
+          acc += w * x[s];
+        }
+        const float o = denom > 0.f ? acc / denom : 0.f;
+        const int g = r / a.M, m = r % a.M;
+        const int64_t h = hk * a.groups + g;
+        uint16_t* dst = a.final_o + b * a.o_sb + h * a.o_sh + static_cast<int64_t>(m) * a.o_sm + d;
+        if constexpr (BF16) {
+          const __nv_bfloat16 v = __float2bfloat16_rn(o);
+          *dst = *reinterpret_cast<const uint16_t*>(&v);
+        } else {
+          const __half v = __float2half_rn(o);
+          *dst = *reinterpret_cast<const uint16_t*>(&v);
+        }
+        if (d == 0) a.final_lse[(static_cast<int64_t>(b) * a.Hq + h) * a.M + m] = denom > 0.f ? mx + logf(denom) : -INFINITY;
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();  // no block's shared memory goes before block 0 has read it
+  }
 }
 
 template <int D, int R>
 int launch_rows(const DecodeArgs& a, bool bf16, unsigned grid, cudaStream_t stream) {
-  return launch(CHAINED, bf16 ? decode_partial_kernel<D, R, true> : decode_partial_kernel<D, R, false>, dim3(grid),
+  const LaunchForm form{true, a.final_o != nullptr ? static_cast<unsigned>(a.num_splits) : 1u};
+  return launch(form, bf16 ? decode_partial_kernel<D, R, true> : decode_partial_kernel<D, R, false>, dim3(grid),
                 DEC_THREADS, 0, stream, a);
 }
 

@@ -11,6 +11,9 @@ namespace b200attn {
 #define B200ATTN_DECODE_MAX_ROWS 2
 #endif
 constexpr int DECODE_MAX_ROWS = B200ATTN_DECODE_MAX_ROWS;
+// Up to this many splits of a (batch, KV head) are one cluster that merges them itself, without partial results in
+// global memory and without the combine kernel.
+constexpr int DECODE_MAX_CLUSTER = 8;
 // Resident CTAs per SM the streaming kernel is compiled for (its minimum-blocks launch bound).
 constexpr int decode_resident_ctas(int rows) { return rows <= 1 ? 3 : 2; }
 
@@ -23,7 +26,7 @@ struct DecodeArgs {
   int64_t v_sb, v_sh, v_sn;
   float* part_o;             // [B, Hq, num_splits, M, D] fp32, normalised within the split
   float* part_lse;           // [B, Hq, num_splits, M] natural-log normaliser of the split
-  uint16_t* final_o;         // non-null (with num_splits == 1): write the result directly
+  uint16_t* final_o;         // non-null (num_splits up to DECODE_MAX_CLUSTER): write the result directly
   float* final_lse;
   int64_t o_sb, o_sh, o_sm;
   int B, Hq, Hkv, M, N, groups;
