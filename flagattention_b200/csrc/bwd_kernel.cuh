@@ -540,7 +540,9 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
           // decisions cached by the forward (see DropoutCtx::keep_mask)
           const uint32_t* mk = args.drop.keep_mask + (static_cast<int64_t>(b) * args.Hq + h) * args.drop.mask_words * args.M;
           if constexpr (MODE == MODE_Q) {
-            keep_bits = row < args.M ? mk[static_cast<int64_t>(col0 >> 5) * args.M + row] : 0u;
+            // (the last step's second half may lie behind the last word)
+            keep_bits = (row < args.M && (col0 >> 5) < args.drop.mask_words)
+                            ? mk[static_cast<int64_t>(col0 >> 5) * args.M + row] : 0u;
           } else {
             // the warp's 32 key rows share one word index; lane c fetches the word of query
             // col0 + keep_index_of(c) (bit l = key keep_index_of(l) of the warp), and a 32 x 32 bit transpose

@@ -15,6 +15,9 @@ pytestmark = pytest.mark.gpu
     (1, 3, 128, 129, 128, True, (1 << 32) - 8000),  # the counter's low word wraps inside a run of 32
     (1, 2, 513, 640, 32, True, (1 << 31) - 40),     # 32-bit counters that run past 2^31
     (70000, 1, 16, 16, 16, True, 1 << 33),          # more heads than the grid's second dimension holds
+    (2, 3, 640, 1, 128, False, 0),                  # the dQ pass: one word, none behind it for the step's second half
+    (2, 3, 640, 90, 64, False, 0),                  # ... three words, the fourth is the next head's
+    (2, 3, 640, 97, 16, True, 0),                   # ... and four, one key in the last
 ])
 def test_cached_decisions_equal_drawn_decisions(B, H, M, N, D, causal, offset, monkeypatch):
     q, k, v, do = make_qkv(B, H, H, M, N, D, torch.float16, seed=3, requires_grad=True)
