@@ -37,9 +37,10 @@ __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
   f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
 }
 
+// (an ordinary load, not .nc: K and V may be what the previous kernel of the stream wrote, see pdl_wait())
 __device__ __forceinline__ uint4 ldg_stream(const uint16_t* p) {
   uint4 r;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
                : "l"(p));
   return r;
@@ -97,7 +98,7 @@ decode_partial_kernel(const DecodeArgs a) {
   // Element offsets of key n's row in K and V.
   auto row_offsets = [&](int n, int64_t& ko, int64_t& vo) {
     if (paged) {
-      const int64_t blk = __ldg(table + (n >> a.block_shift));
+      const int64_t blk = table[n >> a.block_shift];
       const int64_t r = n & block_mask;
       ko = blk * a.k_sb + r * a.k_sn;
       vo = blk * a.v_sb + r * a.v_sn;

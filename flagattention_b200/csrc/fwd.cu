@@ -195,13 +195,13 @@ namespace b200attn {
 // LSE[row] = max + log(sum_s w_s). One block of 128 threads per (b, h, m) row. The splits'
 // log-normalisers are read, reduced to their maximum and turned into weights by all threads in
 // parallel (kept in shared memory for the first 1024 splits); then thread d accumulates feature d
-// over the splits with independent, unrolled loads. (Three dependent loops over the splits per thread
+// over the splits with independent, unrolled loads. The partials are read at L2: this kernel may be resident while they are
+// still being written and while the previous combine caches the same scratch in L1 (see pdl_wait()). (Three dependent loops over the splits per thread
 // made this kernel as long as the partial pass itself on decode shapes.)
 template <bool BF16>
 __global__ void __launch_bounds__(128)
-splitkv_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse,
-                       void* __restrict__ o, float* __restrict__ lse, int64_t o_sb,
-                       int64_t o_sh, int64_t o_sm, int H, int M, int D, int S) {
+splitkv_combine_kernel(const float* part_o, const float* part_lse, void* o, float* lse, int64_t o_sb, int64_t o_sh,
+                       int64_t o_sm, int H, int M, int D, int S) {
   constexpr int CACHED = 1024;
   __shared__ float w_sh[CACHED];
   __shared__ float red[4];
@@ -227,14 +227,14 @@ splitkv_combine_kernel(const float* __restrict__ part_o, const float* __restrict
   };
   float mx = -INFINITY;
   for (int s = tid; s < S; s += 128) {
-    const float x = l[static_cast<int64_t>(s) * M];
+    const float x = __ldcg(l + static_cast<int64_t>(s) * M);
     if (s < CACHED) w_sh[s] = x;
     mx = fmaxf(mx, x);
   }
   mx = block_reduce(mx, true);
   float part = 0.f;
   for (int s = tid; s < S; s += 128) {
-    const float x = s < CACHED ? w_sh[s] : l[static_cast<int64_t>(s) * M];
+    const float x = s < CACHED ? w_sh[s] : __ldcg(l + static_cast<int64_t>(s) * M);
     const float w = (mx == -INFINITY) ? 0.f : expf(x - mx);
     if (s < CACHED) w_sh[s] = w;
     part += w;
@@ -248,8 +248,8 @@ splitkv_combine_kernel(const float* __restrict__ part_o, const float* __restrict
 #pragma unroll 8
     for (int s = 0; s < S; ++s) {
       const float w = s < CACHED ? w_sh[s]
-                                 : ((mx == -INFINITY) ? 0.f : expf(l[static_cast<int64_t>(s) * M] - mx));
-      acc += w * po[s * step];
+                                 : ((mx == -INFINITY) ? 0.f : expf(__ldcg(l + static_cast<int64_t>(s) * M) - mx));
+      acc += w * __ldcg(po + s * step);
     }
     const float out = denom > 0.f ? acc / denom : 0.f;
     uint16_t* dst = static_cast<uint16_t*>(o) + b * o_sb + h * o_sh + m * o_sm + d;

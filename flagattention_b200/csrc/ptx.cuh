@@ -43,6 +43,11 @@ __device__ __forceinline__ bool elect_one() {
 // this one not completing before its predecessor. pdl_trigger() lets the next kernel start once every block of this
 // one has called it; a kernel that allocates TMEM calls it after the allocation, or a successor's block on the same
 // SM could take the columns and wait for this kernel for ever. Both do nothing in an ordinary launch.
+// A chained kernel is resident while a chained predecessor, which triggers early, still writes. What such a predecessor
+// may have written (any input of an operator, partial results) is therefore not read-only for the kernel's lifetime: no
+// __ldg(), ld.global.nc or const __restrict__ on it, whose loads may be served from a cache that nobody invalidates or
+// moved ahead of the wait. (The cache of dropout decisions is read with __ldg(): the kernel that fills it does not
+// trigger, so its reader starts behind it.)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
