@@ -69,6 +69,7 @@ struct BwdArgs {
   int32_t* status;
   float* dq_acc;        // FUSED: [B, Hq, M, D] fp32, zero before the launch
   int out_tma;          // the 16-bit results leave through shared memory and TMA stores (tmO1, tmO2)
+  int kv_split;         // MODE_KV: blocks of the cluster that shares a key block (see bwd_kv_split()), 1: no cluster
   int out2_accumulate;  // MODE_KV: out2 (dV) already holds a 16-bit gradient that this pass adds to
 };
 
@@ -104,7 +105,9 @@ struct BwdSmem {
   static constexpr int THREADS = 32 * (4 * GROUPS + 2 + DQ_WARPS);
 };
 
-template <int D, bool BF16, bool DROPOUT, int MODE, bool FUSED = false>
+// SHARED (MODE_KV): args.kv_split > 1. (A template parameter: as a run-time choice it cost launches that share nothing
+// a per cent.)
+template <int D, bool BF16, bool DROPOUT, int MODE, bool FUSED = false, bool SHARED = false>
 __global__ void __launch_bounds__((BwdSmem<D, MODE, FUSED>::THREADS), (BwdSmem<D, MODE, FUSED>::BLOCKS))
 bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUtensorMap tmA2,
            const __grid_constant__ CUtensorMap tmB1, const __grid_constant__ CUtensorMap tmB2,
@@ -161,7 +164,12 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
   // Row block, the heads it loops over and its column range [col_lo, col_hi) in steps of 64.
   int r0, h_first, n_heads, hk, col_lo, col_hi;
   const int grid_heads = MODE == MODE_KV ? args.Hkv : args.Hq;
-  const BlockCoord bc = decode_block(blockIdx.x, args.B * grid_heads, args.n_zblocks, args.grid_chunk);
+  // MODE_KV: the kv_split blocks of a cluster share the key block's steps; their dK and dV are summed at the end.
+  static_assert(!SHARED || MODE == MODE_KV, "key blocks are shared in the dK/dV pass");
+  const int kv_split = SHARED ? args.kv_split : 1;
+  const int kv_rank = SHARED ? static_cast<int>(blockIdx.x) % kv_split : 0;
+  const int unit = SHARED ? static_cast<int>(blockIdx.x) / kv_split : static_cast<int>(blockIdx.x);
+  const BlockCoord bc = decode_block(unit, args.B * grid_heads, args.n_zblocks, args.grid_chunk);
   const int b = bc.bh / grid_heads;
   const int grid_h = bc.bh % grid_heads;
   if constexpr (MODE == MODE_Q) {
@@ -187,7 +195,17 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
     col_hi = (args.causal && args.d_max < BAND_INF) ? min(args.M, max(0, r0 + 127 - P_SEQ + args.d_max)) : args.M;
   }
   const int steps_per_head = col_hi > col_lo ? cdiv(col_hi - col_lo, STEP) : 0;
-  const int T = steps_per_head * n_heads;
+  // Steps of this block: all of them, or the share [i_first, i_first + T) of the cluster's.
+  int i_first = 0, T = steps_per_head * n_heads;
+  if constexpr (SHARED) {
+    i_first = static_cast<int>(static_cast<int64_t>(T) * kv_rank / kv_split);
+    T = static_cast<int>(static_cast<int64_t>(T) * (kv_rank + 1) / kv_split) - i_first;
+  }
+  if constexpr (MODE == MODE_KV) {
+    // start inside the first head of the share (the loops below count steps from there)
+    if (i_first > 0) h_first += i_first / steps_per_head;
+  }
+  const int i_skip = i_first > 0 ? i_first % steps_per_head : 0;
 
   if (threadIdx.x == 0) {
     mbar_init(a_full, 1);
@@ -242,8 +260,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
       }
       for (int i = 0; i < T; ++i) {
         const int st = i % STAGES;
-        const int hh = i / steps_per_head;
-        const int col = col_lo + (i - hh * steps_per_head) * STEP;
+        const int hh = (i + i_skip) / steps_per_head;
+        const int col = col_lo + (i + i_skip - hh * steps_per_head) * STEP;
         const int b_head = MODE == MODE_Q ? hk : h_first + hh;
         if (!wait(&b_empty[st], ((i / STAGES) & 1) ^ 1)) { fail(ST_WAIT_EMPTY); break; }
         uint8_t* stage = sB + st * Sm::STAGE_BYTES;
@@ -414,8 +432,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
       const int d = (warp & 3) * 32 + lane;  // feature index = TMEM lane
       for (int i = 0; i < T; ++i) {
         const int buf = buf_of(i);
-        const int hh = i / steps_per_head;
-        const int col = col_lo + (i - hh * steps_per_head) * STEP;
+        const int hh = (i + i_skip) / steps_per_head;
+        const int col = col_lo + (i + i_skip - hh * steps_per_head) * STEP;
         {
           // The four warps decide together whether to go on: they meet at named barriers below, so
           // one of them leaving alone would strand the others there. Each warp's own wait is bounded,
@@ -508,8 +526,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
     for (int i = 0; i < T; ++i) {
       const int st = i % STAGES;
       const int buf = buf_of(i);
-      const int hh = i / steps_per_head;
-      const int col0 = col_lo + (i - hh * steps_per_head) * STEP + wg * HALF;  // first column of this group
+      const int hh = (i + i_skip) / steps_per_head;
+      const int col0 = col_lo + (i + i_skip - hh * steps_per_head) * STEP + wg * HALF;  // first column of this group
       const int h = h_first + hh;
       const uint32_t t1_addr = tmem_base + lane_base + BUF_BASE + buf * BUF_COLS;
       // Dropout decisions for this thread's 32 (row, column) pairs of the step, generated before the
@@ -730,6 +748,24 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
         for (int g = 1; g < GROUPS; ++g) tot_sum += red[(g - 1) * 128 + row_local];
         args.tot[(static_cast<int64_t>(b) * args.Hq + h_first) * args.N + row] = tot_sum;
       }
+    } else if constexpr (SHARED) {
+      // Shared key block: this block's dK and dV go to shared memory in fp32, [accumulator][column][row], over the
+      // resident tiles and the ring (all their readers have completed); summed below.
+      tc_fence_after();
+      float* part = reinterpret_cast<float*>(smem);
+#pragma unroll
+      for (int acc = 0; acc < N_ACC; ++acc) {
+#pragma unroll
+        for (int c = wg * (D / GROUPS); c < (wg + 1) * (D / GROUPS); c += 8) {
+          uint32_t o[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+          if (T > 0 && ok) {
+            tmem_ld8(tmem_base + lane_base + acc * D + c, o);
+            tmem_wait_ld();
+          }
+#pragma unroll
+          for (int x = 0; x < 8; ++x) part[(acc * D + c + x) * 128 + row_local] = __uint_as_float(o[x]);
+        }
+      }
     } else if (args.out_tma) {
       // Each thread scales and rounds its part of a row of every accumulator into the (now dead) resident
       // tile of the same index, in the swizzled layout of the output tensor map; one thread then
@@ -869,6 +905,48 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUt
     }
   }
 
+  if constexpr (SHARED) {
+    // Sum of the cluster's dK and dV in the order of the ranks; rank r finishes columns [r, r + 1) D / kv_split.
+    // (Every thread comes here whatever became of its waits.)
+    static_assert(N_ACC * D * 128 * 4 <= Sm::DS_OFFSET, "the fp32 sums lie over the resident tiles and the ring");
+    __syncwarp();
+    cluster_sync_all();
+    const int units = D / kv_split / 8;  // groups of 8 columns per accumulator
+    const int r = static_cast<int>(threadIdx.x) & 127;
+    if (threadIdx.x < 128 * GROUPS && r0 + r < args.N) {
+      for (int u = static_cast<int>(threadIdx.x) >> 7; u < N_ACC * units; u += GROUPS) {
+        const int acc = u / units, c = kv_rank * (D / kv_split) + (u - acc * units) * 8;
+        const uint32_t at = smem_u32(smem) + ((acc * D + c) * 128 + r) * 4;
+        float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int k = 0; k < kv_split; ++k) {
+          const uint32_t peer = cluster_map(at, k);
+#pragma unroll
+          for (int x = 0; x < 8; ++x) f[x] += cluster_load(peer + x * 512);
+        }
+        const float scale = acc == 0 ? args.sm_scale : DROPOUT ? args.drop.inv_keep : 1.0f;
+#pragma unroll
+        for (int x = 0; x < 8; ++x) f[x] *= scale;
+        uint16_t* out = acc == 0 ? static_cast<uint16_t*>(args.out1) + b * args.out1_sb + hk * args.out1_sh +
+                                       static_cast<int64_t>(r0 + r) * args.out1_sr + c
+                                 : static_cast<uint16_t*>(args.out2) + b * args.out2_sb + hk * args.out2_sh +
+                                       static_cast<int64_t>(r0 + r) * args.out2_sr + c;
+        if (acc == 1 && args.out2_accumulate) {
+          const uint4 pv = *reinterpret_cast<const uint4*>(out);
+          const uint32_t w[4] = {pv.x, pv.y, pv.z, pv.w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 g = unpack2<BF16>(w[i]);
+            f[2 * i] += g.x;
+            f[2 * i + 1] += g.y;
+          }
+        }
+        *reinterpret_cast<uint4*>(out) = make_uint4(pack2<BF16>(f[0], f[1]), pack2<BF16>(f[2], f[3]),
+                                                    pack2<BF16>(f[4], f[5]), pack2<BF16>(f[6], f[7]));
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();  // no block's shared memory goes before its peers have read it
+  }
   tc_fence_before();
   __syncthreads();
   __syncwarp();

@@ -16,9 +16,12 @@ struct BwdLaunch {
   cudaStream_t stream;
 };
 
-template <int D, bool BF16, bool DROPOUT, int MODE, bool FUSED = false>
+template <int D, bool BF16, bool DROPOUT, int MODE, bool FUSED = false, bool SHARED = false>
 int launch_bwd_variant(const BwdLaunch& L) {
-  auto kernel = bwd_kernel<D, BF16, DROPOUT, MODE, FUSED>;
+  if constexpr (MODE == MODE_KV && !SHARED) {
+    if (L.args.kv_split > 1) return launch_bwd_variant<D, BF16, DROPOUT, MODE, FUSED, true>(L);
+  }
+  auto kernel = bwd_kernel<D, BF16, DROPOUT, MODE, FUSED, SHARED>;
   constexpr int smem = BwdSmem<D, MODE, FUSED>::TOTAL;
   static PerDeviceOnce attr_once;  // one per kernel variant
   const int rc = attr_once.run([&]() -> int {
@@ -26,8 +29,9 @@ int launch_bwd_variant(const BwdLaunch& L) {
     return B200ATTN_OK;
   });
   if (rc) return rc;
-  return launch(LaunchForm{}, kernel, L.grid, BwdSmem<D, MODE, FUSED>::THREADS, smem, L.stream, L.tmA1, L.tmA2, L.tmB1, L.tmB2,
-                L.tmO1, L.tmO2, L.args);
+  const LaunchForm form{false, SHARED ? static_cast<unsigned>(L.args.kv_split) : 1u};
+  return launch(form, kernel, L.grid, BwdSmem<D, MODE, FUSED>::THREADS, smem, L.stream, L.tmA1, L.tmA2, L.tmB1, L.tmB2, L.tmO1,
+                L.tmO2, L.args);
 }
 
 template <int D>

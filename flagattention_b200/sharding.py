@@ -4,10 +4,8 @@ The operator is independent per (batch, KV head): all query heads that share a K
 rank, so dK/dV need no cross-rank reduction. ``unit_range`` assigns each rank a contiguous range
 of the ``B * Hkv`` units; ``shard`` returns the matching views of q, k, v (and anything shaped
 like q), one piece per batch the range touches. One process per GPU runs its pieces through the
-ordinary ``flash_attention``; outputs, dK and dV are bit-identical to the corresponding slices of a
-single-GPU run, and so is dQ under ``torch.use_deterministic_algorithms(True)`` (by default its fp32 sums
-have no fixed order at head dimensions 32 and up). The exception are pieces with so few query rows that
-the forward splits their keys (``split_kv.choose_num_splits``, which counts batch and heads).
+ordinary ``flash_attention``; results are bit-identical to the corresponding slices of a
+single-GPU run.
 """
 from __future__ import annotations
 
