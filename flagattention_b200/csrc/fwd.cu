@@ -214,6 +214,14 @@ splitkv_combine_kernel(const float* part_o, const float* part_lse, void* o, floa
   const int64_t b = bh / H;
   const float* l = part_lse + bh * S * M + m;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  // The first splits' values are on their way while the weights are formed; later ones come up to sixteen at a time.
+  constexpr int AHEAD = 4, BATCH = 16;
+  const int d = tid;
+  const float* po = part_o + (bh * S * M + m) * D + d;
+  const int64_t step = static_cast<int64_t>(M) * D;
+  float ahead[AHEAD];
+#pragma unroll
+  for (int s = 0; s < AHEAD; ++s) ahead[s] = d < D && s < S ? __ldcg(po + s * step) : 0.f;
   auto block_reduce = [&](float x, bool is_max) -> float {
 #pragma unroll
     for (int off = 16; off >= 1; off >>= 1) {
@@ -240,16 +248,29 @@ splitkv_combine_kernel(const float* part_o, const float* part_lse, void* o, floa
     part += w;
   }
   const float denom = block_reduce(part, false);
-  const int d = tid;
   if (d < D) {
     float acc = 0.f;
-    const float* po = part_o + (bh * S * M + m) * D + d;
-    const int64_t step = static_cast<int64_t>(M) * D;
-#pragma unroll 8
-    for (int s = 0; s < S; ++s) {
-      const float w = s < CACHED ? w_sh[s]
-                                 : ((mx == -INFINITY) ? 0.f : expf(__ldcg(l + static_cast<int64_t>(s) * M) - mx));
-      acc += w * __ldcg(po + s * step);
+    auto weight = [&](int s) -> float {
+      return s < CACHED ? w_sh[s] : mx == -INFINITY ? 0.f : expf(__ldcg(l + static_cast<int64_t>(s) * M) - mx);
+    };
+#pragma unroll
+    for (int s = 0; s < AHEAD; ++s)
+      if (s < S) acc += weight(s) * ahead[s];
+    int s0 = AHEAD;
+    for (; s0 + BATCH <= S; s0 += BATCH) {
+      float x[BATCH];
+#pragma unroll
+      for (int i = 0; i < BATCH; ++i) x[i] = __ldcg(po + (s0 + i) * step);
+#pragma unroll
+      for (int i = 0; i < BATCH; ++i) acc += weight(s0 + i) * x[i];
+    }
+    for (; s0 < S; s0 += 4) {
+      float x[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = s0 + i < S ? __ldcg(po + (s0 + i) * step) : 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (s0 + i < S) acc += weight(s0 + i) * x[i];
     }
     const float out = denom > 0.f ? acc / denom : 0.f;
     uint16_t* dst = static_cast<uint16_t*>(o) + b * o_sb + h * o_sh + m * o_sm + d;
