@@ -6,8 +6,9 @@ this library's kernels.
 bands of the distance, so the row's softmax is the normaliser-weighted merge of two band-limited
 attentions: the forward runs the forward kernel once per (q, k) pair with the band mask of its region,
 the near region into an fp32 partial output and log-normaliser (``b200attn_fwd`` with ``band``), the far
-region combining its rows with them in its epilogue (``b200attn_fwd_merge``, the algebra of the split-KV
-combine, rounding straight into the output). The backward runs the backward
+region combining its rows with them in its epilogue (``b200attn_fwd_merge``) or writing partial results too,
+which ``b200attn_merge_partial_store`` merges; both are the algebra of the split-KV combine and round
+straight into the output. The backward runs the backward
 kernels once per pair with the same bands, both on the merged log-normaliser and on ``delta`` of the
 merged output; each call yields its pair's dQ and dK, and the two dV contributions are added.
 """
@@ -18,7 +19,7 @@ import math
 import torch
 
 from . import _lib
-from .flash import _status_word, _tma_ready
+from .flash import _sm_count, _status_word, _tma_ready
 
 _SUPPORTED_HEAD_DIMS = (16, 32, 64, 128)
 
@@ -28,6 +29,16 @@ def _bands(w: int, causal: bool):
     near = (0 if causal else _lib.BAND_OPEN_MIN, w)
     far = (max(w, 0) if causal else w, _lib.BAND_OPEN_MAX)
     return near, far
+
+
+def _merges_in_epilogue(pairs: int, M: int, D: int, num_sms: int) -> bool:
+    """Whether the far region's forward combines its rows with the near region's result in its epilogue, or both regions
+    leave fp32 partial results that a kernel of its own merges. The epilogue saves that kernel and a partial result, and
+    reads the other one a row per thread while the tensor cores wait: at D = 128 it gains (B4 H16 2048 causal 174 -> 168
+    us, B16 H16 900 262 -> 248), at D <= 64, where a tile's products are half as long, it loses (B2 H32 1841 causal D64
+    138 -> 149, B4 H16 2048 D32 113 -> 118) unless all work items run at once and the launch is what shows (B3 H4 397
+    D64 66 -> 53)."""
+    return D == 128 or pairs * -(-M // 256) <= num_sms
 
 
 class PiecewiseAttentionFunction(torch.autograd.Function):
@@ -55,21 +66,29 @@ class PiecewiseAttentionFunction(torch.autograd.Function):
             stream = _lib.current_stream_ptr(device)
             status = _status_word(device)
             near, far = _bands(w, bool(causal))
-            # The near region's result stays in fp32; the far region's forward combines its own rows with it.
-            o_near = torch.empty((B, H, M, D), dtype=torch.float32, device=device)
-            l_near = torch.empty((B, H, M), dtype=torch.float32, device=device)
+
+            def empty32(*shape):
+                return torch.empty(shape, dtype=torch.float32, device=device)
+
+            def region(q, k, band, out, norm):
+                return _lib.FwdParams(
+                    _lib.tensor4(q), _lib.tensor4(k), _lib.tensor4(v), _lib.tensor4(out), norm.data_ptr(),
+                    B, H, H, M, N, D, dt, _lib.dtype_code(out.dtype), int(bool(causal)), float(sm_scale),
+                    0.0, 0, 0, status.data_ptr(), 1, *band)
+
             o = torch.empty_like(q1)
-            L = torch.empty((B, H, M), dtype=torch.float32, device=device)
-            fp = _lib.FwdParams(
-                _lib.tensor4(q1), _lib.tensor4(k1), _lib.tensor4(v), _lib.tensor4(o_near), l_near.data_ptr(),
-                B, H, H, M, N, D, dt, _lib.dtype_code(torch.float32), int(bool(causal)), float(sm_scale),
-                0.0, 0, 0, status.data_ptr(), 1, *near)
-            _lib.check(lib.b200attn_fwd(fp, stream), "b200attn_fwd")
-            fp = _lib.FwdParams(
-                _lib.tensor4(q2), _lib.tensor4(k2), _lib.tensor4(v), _lib.tensor4(o), L.data_ptr(),
-                B, H, H, M, N, D, dt, dt, int(bool(causal)), float(sm_scale),
-                0.0, 0, 0, status.data_ptr(), 1, *far)
-            _lib.check(lib.b200attn_fwd_merge(fp, o_near.data_ptr(), l_near.data_ptr(), stream), "b200attn_fwd_merge")
+            o_near, l_near = empty32(B, H, M, D), empty32(B, H, M)
+            _lib.check(lib.b200attn_fwd(region(q1, k1, near, o_near, l_near), stream), "b200attn_fwd")
+            if _merges_in_epilogue(B * H, M, D, _sm_count(device)):
+                L = empty32(B, H, M)
+                _lib.check(lib.b200attn_fwd_merge(region(q2, k2, far, o, L), o_near.data_ptr(), l_near.data_ptr(), stream),
+                           "b200attn_fwd_merge")
+            else:
+                o_far, l_far, L = empty32(B, H, M, D), empty32(B, H, M), l_near
+                _lib.check(lib.b200attn_fwd(region(q2, k2, far, o_far, l_far), stream), "b200attn_fwd")
+                _lib.check(lib.b200attn_merge_partial_store(o_near.data_ptr(), L.data_ptr(), o_far.data_ptr(), l_far.data_ptr(),
+                                                            B, H, M, D, _lib.tensor4(o), dt, stream),
+                           "b200attn_merge_partial_store")
         ctx.save_for_backward(q1, k1, q2, k2, v, o, L)
         ctx.sm_scale = sm_scale
         ctx.causal = bool(causal)

@@ -4,7 +4,7 @@ contracts differently."""
 import pytest
 import torch
 
-from flagattention_b200 import _lib
+from flagattention_b200 import _lib, piecewise, piecewise_attention
 from gpu_util import device, make_qkv
 
 pytestmark = pytest.mark.gpu
@@ -51,3 +51,21 @@ def test_against_the_merge_kernel(M, N, near, far, D, dtype, layout):
     # it is rounded to 16 bits: half an ulp of P on each side, times the largest |v|.
     slack = ulp * v.float().abs().max() if far[1] == 2 ** 31 - 1 and far[0] == -2 ** 31 else 1e-6
     assert (got.float() - want.float()).abs().le(ulp * want.float().abs() + slack).all()
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+def test_both_ways_of_the_operator(D, causal, monkeypatch):
+    """More work items than SMs, where head dimensions up to 64 merge in a kernel of their own."""
+    inputs = [torch.randn(3, 50, 257, D, device=device(), dtype=torch.float16, generator=torch.Generator(device()).manual_seed(i))
+              for i in range(5)]
+    assert piecewise._merges_in_epilogue(150, 257, D, 148) == (D == 128) and piecewise._merges_in_epilogue(74, 257, D, 148)
+    got = {}
+    for epilogue in (False, True):
+        monkeypatch.setattr(piecewise, "_merges_in_epilogue", lambda *args: epilogue)
+        leaves = [t.clone().requires_grad_() for t in inputs]
+        o = piecewise_attention(*leaves, 100, causal=causal)
+        got[epilogue] = (o.detach(),) + torch.autograd.grad(o, leaves[4], inputs[0])
+    for a, b in zip(got[False], got[True]):   # neighbouring fp16 numbers where the compiler contracts differently
+        a, b = a.float(), b.float()
+        assert (a - b).abs().le(2.0 ** -10 * b.abs() + 1e-4 * b.abs().max()).all()
