@@ -461,9 +461,19 @@ static int run_splitkv(const b200attn_splitkv_params* p, const PagedKV* paged, v
     a.bt_stride = paged->bt_stride;
     a.context_lens = paged->context_lens;
     a.block_shift = paged->block_shift;
-    // (one thread each; with at most one block per SM the order is of no use and ranking costs 1.5 us)
-    const int64_t entries = static_cast<int64_t>(p->B) * cta_splits;
-    a.sort_entries = packed && entries <= 384 && entries * p->Hkv > sm_count() ? static_cast<int>(entries) : 0;
+    // Longest first: sequences of a batch differ in length, and in their given order the last blocks run alone. 32
+    // sequences of 1024 to 4096 keys, Hq64 Hkv8 D128: 90.4 -> 76.7 us; 24 geometrically spread up to 4096: 56.1 -> 42.4.
+    // Ranking takes one thread per entry and about 1.5 us of every block, so not where
+    // - there is a block per SM or less;
+    // - a sequence is cut into more than three: most entries are then equally long and run in step, all of them starting
+    //   up at once (15 sequences up to 14333 keys, Hq64 Hkv8 D128, six cuts: 117.1 given, 124.5 sorted);
+    // - many short blocks follow one another: what the order gains is part of one block, what it costs is paid by each
+    //   (128 sequences up to 1000 keys, Hq64 Hkv16 D64, 14 rounds of 8 tiles: 188.1 given, 197.5 sorted; Hq32 Hkv4, 3.5
+    //   rounds: 58.2, 59.5; D128, 3.5 rounds: 74.6, 74.4). The line is at 160 tile columns a round.
+    const int64_t entries = static_cast<int64_t>(p->B) * cta_splits, items = entries * p->Hkv;
+    const bool pays = items > sm_count() && cta_splits <= 3 &&
+                      static_cast<int64_t>(a.tiles_per_split) * p->D * sm_count() >= 160 * items;
+    a.sort_entries = packed && entries <= 384 && pays ? static_cast<int>(entries) : 0;
   }
   a.ring_stages = p->D == 128 ? FwdSmem<128>::DUAL_STAGES
                   : p->D == 64 ? FwdSmem<64>::DUAL_STAGES

@@ -77,9 +77,8 @@ struct FwdArgs {
   const int32_t* context_lens;
   int block_shift;
   int sort_entries;                 // > 0 (paged, packed): the (sequence, split) entries of the launch, at most one per
-                                    // thread; they are taken longest first. Sequences of a batch differ in length, and in
-                                    // their given order the last blocks run alone: 32 sequences of 1024 to 4096 keys,
-                                    // Hq64 Hkv8 D128: 92.5 -> 78 us.
+                                    // thread; they are taken longest first unless all sequences have the same number of
+                                    // tiles (see run_splitkv() in fwd.cu)
   int B, Hq, Hkv, M, N, groups;
   int causal, o_fp32;               // causal: some band limit below is finite (enables the masking code)
   // Visibility band: query m sees key n iff d_min <= m + (N - M) - n < d_max. Plain causal masking is
@@ -205,6 +204,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     int n_sub[2];    // SPLIT64: number of 64-key sub-steps each query tile runs
     int n_max;       // number of K/V tiles the CTA streams
   };
+  bool longest_first = false;  // sort_entries, and the sequences differ in length
   auto get_item = [&](int id) -> Item {
     Item it;
     const BlockCoord bc = args.order.decode(id);
@@ -212,8 +212,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     it.split = bc.z - z_row * args.num_splits;
     const int m_blk = args.div_splits.div(args.n_zblocks) - 1 - z_row;  // longest first
     it.b = args.div_heads.div(bc.bh);
-    const int head = args.sort_entries > 0 ? id % grid_heads : bc.bh - it.b * grid_heads;
-    if (args.sort_entries > 0) {
+    const int head = longest_first ? id % grid_heads : bc.bh - it.b * grid_heads;
+    if (longest_first) {
       it.b = *my_entry / args.num_splits;
       it.split = *my_entry - it.b * args.num_splits;
     }
@@ -294,22 +294,28 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     int* tiles = reinterpret_cast<int*>(sQ);  // (no load has been issued yet)
     const int e = static_cast<int>(threadIdx.x), n = args.sort_entries;
     int mine = 0;
+    bool differs = false;
     if (e < n) {
       const int seq = e / args.num_splits, first = (e - seq * args.num_splits) * args.tiles_per_split;
-      mine = max(0, min(cdiv(args.context_lens[seq], BLOCK) - first, args.tiles_per_split));
+      const int length = cdiv(args.context_lens[seq], BLOCK);
+      differs = length != cdiv(args.context_lens[0], BLOCK);
+      mine = max(0, min(length - first, args.tiles_per_split));
       tiles[e] = mine;
     }
-    __syncthreads();
-    if (e < n) {
-      int rank = 0;
-      for (int j = 0; j < n; ++j) {
-        const int other = tiles[j];
-        rank += (other > mine || (other == mine && j < e)) ? 1 : 0;
-      }
-      if (rank == static_cast<int>(blockIdx.x) / grid_heads) *my_entry = e;
-    }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the Q tile is loaded over `tiles`
-    __syncthreads();
+    longest_first = __syncthreads_or(differs);
+    if (longest_first) {
+      if (e < n) {
+        int rank = 0;
+        for (int j = 0; j < n; ++j) {
+          const int other = tiles[j];
+          rank += (other > mine || (other == mine && j < e)) ? 1 : 0;
+        }
+        if (rank == static_cast<int>(blockIdx.x) / grid_heads) *my_entry = e;
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncthreads();
+    }
   }
 
   auto fail = [&](int32_t code) {

@@ -13,8 +13,10 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("splits", [1, 2, 4])
 @pytest.mark.parametrize("lens", [
     [1], [700, 700, 700],                       # nothing to order, nothing but ties
+    [641 + i for i in range(12)], [640, 641, 640, 640, 640, 640],   # as many tiles each, one more in one of them
     [5, 1500, 128, 129, 1024, 1, 640],          # one key, edges of a 128-key tile, empty last splits
     [(37 * i) % 300 + 1 for i in range(192)],   # with two CTA splits as many entries as threads
+    [(37 * i) % 900 + 1000 for i in range(192)],   # ... of blocks long enough to be ordered
     [(37 * i) % 300 + 1 for i in range(385)],   # more: the given order
 ])
 def test_each_sequence_as_alone(lens, splits, D, block):
