@@ -9,6 +9,7 @@
 #include <ATen/ATen.h>
 #include <ATen/FuncTorchTLS.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -85,9 +86,23 @@ bool ready(const at::Tensor& x, int dims) {
   return true;
 }
 
+// Whether a functorch transform is active on this thread. A thread that has ever used functorch, also through
+// torch.compile, keeps its functorch state; the state itself knows whether a transform is active and then refuses C++
+// autograd functions. (The key test only spares the exception in the usual case.)
+bool transform_active() {
+  const auto& state = at::functorch::functorchTLSAccessor();
+  if (!state) return false;
+  if (c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode)) return true;
+  try {
+    state->checkSupportsCppAutogradFunction();
+  } catch (const c10::Error&) {
+    return true;
+  }
+  return false;
+}
+
 bool ordinary_mode() {
-  return !at::functorch::functorchTLSAccessor() && !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
-         !torch::jit::tracer::isTracing();
+  return !transform_active() && !c10::impl::TorchDispatchModeTLS::any_modes_set() && !torch::jit::tracer::isTracing();
 }
 
 bool head_dim_ok(int64_t d) { return d == 16 || d == 32 || d == 64 || d == 128; }
@@ -362,7 +377,15 @@ PyObject* split_branch(PyObject*, PyObject* args) {
   return PyBool_FromLong(takes_split_branch(b, h, m, n, sms));
 }
 
+// ordinary_mode(): that rule by itself
+PyObject* mode_is_ordinary(PyObject*, PyObject*) {
+  HANDLE_TH_ERRORS
+  return PyBool_FromLong(ordinary_mode());
+  END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef methods[] = {
+    {"ordinary_mode", &mode_is_ordinary, METH_NOARGS, nullptr},
     {"takes_split_branch", &split_branch, METH_VARARGS, nullptr},
     {"flash", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&attention<false>)), METH_FASTCALL, nullptr},
     {"split_kv", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&attention<true>)), METH_FASTCALL, nullptr},

@@ -72,6 +72,22 @@ def test_forms_that_are_handed_on():
         flash_attention(q[:, :3], k, v)
 
 
+def test_calls_are_taken_after_a_transform_and_a_compilation():
+    """(also what makes the tests below, and in the files behind this one, run the native path)"""
+    host = _lib.host()
+    q, k, v, _ = make_qkv(2, 4, 2, 64, 64, 64, torch.float16, seed=1)
+    lens, tables = torch.tensor([40, 64], device=device(), dtype=torch.int32), torch.zeros(2, 4, device=device(), dtype=torch.int32)
+    cache = torch.randn(3, 2, 16, 64, device=device(), dtype=torch.float16)
+
+    def taken():
+        return [x is not None for x in (host.flash(q, k, v, False, None), host.split_kv(q, k, v, False, None),
+                                        host.paged(q[:, :, 0].contiguous(), cache, cache, lens, tables, 0.125, 64, 0))]
+    torch.func.vmap(lambda x: x + 1)(q)
+    assert taken() == [True] * 3
+    torch.compile(lambda x: x * 2 + 1, backend="eager")(q)
+    assert taken() == [True] * 3
+
+
 def test_gradient_of_another_type_stride_and_only_some_inputs():
     q, k, v, do = make_qkv(1, 4, 4, 160, 160, 64, torch.float16, seed=3)
     k.requires_grad_()

@@ -1,7 +1,9 @@
-"""The native host path's copy of the split-KV rule against the Python one, and that it takes no CPU tensor."""
+"""The native host path's copy of the split-KV rule against the Python one, that it takes no CPU tensor, and in which
+modes of torch it takes calls."""
 import random
 
 import torch
+from torch._subclasses import FakeTensorMode
 
 from flagattention_b200 import _lib
 from flagattention_b200.split_kv import choose_num_splits
@@ -22,3 +24,28 @@ def test_cpu_tensors_are_handed_on():
     host = _lib.host()
     assert host.flash(q, q, q, False, None) is None and host.split_kv(q, q, q, False, None) is None
     assert host.paged(q[0], q, q, torch.ones(2, dtype=torch.int32), torch.zeros(2, 1, dtype=torch.int32), 0.1, 4, 0) is None
+
+
+def test_ordinary_mode_ends_and_comes_back():
+    """Transforms, dispatch modes and tracers are handed on while they are active, and not for the rest of the thread."""
+    ordinary = _lib.host().ordinary_mode
+    x = torch.ones(3)
+    seen = []
+
+    def look(t):
+        seen.append(ordinary())
+        return t * 2
+
+    assert ordinary()
+    torch.func.vmap(look)(x)
+    torch.func.grad(lambda t: look(t).sum())(x)
+    torch.func.jvp(look, (x,), (x,))
+    torch.func.vmap(torch.func.grad(lambda t: look(t).sum()))(torch.ones(2, 3))
+    torch.func.functionalize(look)(x)
+    assert seen == [False] * 5 and ordinary()
+    with FakeTensorMode():
+        assert not ordinary()
+    torch.jit.trace(look, x, check_trace=False)
+    assert seen[5:] == [False] and ordinary()
+    torch.compile(lambda t: t * 2 + 1, backend="eager")(x)
+    assert ordinary()
