@@ -251,9 +251,10 @@ struct FlashAttention : torch::autograd::Function<FlashAttention> {
   }
 };
 
-bool all_tensors(PyObject* const* args, int n) {
+// Exactly torch.Tensor or nn.Parameter: another subclass may define its own results, through __torch_function__ too.
+bool plain_tensors(PyObject* const* args, int n) {
   for (int i = 0; i < n; ++i)
-    if (!THPVariable_Check(args[i])) return false;
+    if (!THPVariable_CheckExact(args[i])) return false;
   return true;
 }
 
@@ -271,7 +272,7 @@ bool scale_of(PyObject* arg, int64_t d, double* out) {
 template <bool SPLIT>
 PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 5 || !all_tensors(args, 3) || !ordinary_mode()) Py_RETURN_NONE;
+  if (n != 5 || !plain_tensors(args, 3) || !ordinary_mode()) Py_RETURN_NONE;
   const at::Tensor &q = THPVariable_Unpack(args[0]), &k = THPVariable_Unpack(args[1]), &v = THPVariable_Unpack(args[2]);
   if (!qkv_ok(q, k, v)) Py_RETURN_NONE;
   const int causal = PyObject_IsTrue(args[3]);
@@ -292,7 +293,7 @@ PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // paged(query, key_cache, value_cache, context_lens, block_tables, attn_scale, max_context_len, num_splits)
 PyObject* paged(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 8 || !all_tensors(args, 5) || !ordinary_mode()) Py_RETURN_NONE;
+  if (n != 8 || !plain_tensors(args, 5) || !ordinary_mode()) Py_RETURN_NONE;
   const at::Tensor &q = THPVariable_Unpack(args[0]), &kc = THPVariable_Unpack(args[1]), &vc = THPVariable_Unpack(args[2]),
                    &lens = THPVariable_Unpack(args[3]), &tables = THPVariable_Unpack(args[4]);
   if (!ready(q, 3) || !ready(kc, 4) || !ready(vc, 4)) Py_RETURN_NONE;

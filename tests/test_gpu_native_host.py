@@ -72,6 +72,20 @@ def test_forms_that_are_handed_on():
         flash_attention(q[:, :3], k, v)
 
 
+class _Named(torch.Tensor):
+    """A subclass without __torch_dispatch__, whose operations return it again."""
+
+
+def test_subclasses_come_back_as_from_python(monkeypatch):
+    q, k, v, _ = make_qkv(2, 4, 2, 64, 64, 64, torch.float16, seed=2)
+    named = q.as_subclass(_Named)
+    x, y = _both(monkeypatch, lambda: flash_attention(named, k, v))
+    assert type(x) is type(y) is _Named and torch.equal(x.as_subclass(torch.Tensor), flash_attention(q, k, v))
+    host = _lib.host()
+    assert host.flash(named, k, v, False, None) is None and host.split_kv(q, k.as_subclass(_Named), v, False, None) is None
+    assert host.flash(torch.nn.Parameter(q), k, v, False, None) is not None
+
+
 def test_calls_are_taken_after_a_transform_and_a_compilation():
     """(also what makes the tests below, and in the files behind this one, run the native path)"""
     host = _lib.host()
