@@ -273,18 +273,23 @@ template <bool SPLIT>
 PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n != 5 || !plain_tensors(args, 3) || !ordinary_mode()) Py_RETURN_NONE;
-  const at::Tensor &q = THPVariable_Unpack(args[0]), &k = THPVariable_Unpack(args[1]), &v = THPVariable_Unpack(args[2]);
+  const at::Tensor q = THPVariable_Unpack(args[0]), k = THPVariable_Unpack(args[1]), v = THPVariable_Unpack(args[2]);
   if (!qkv_ok(q, k, v)) Py_RETURN_NONE;
   const int causal = PyObject_IsTrue(args[3]);
   double scale;
   if (causal < 0 || !scale_of(args[4], q.size(3), &scale)) return nullptr;
-  const c10::cuda::OptionalCUDAGuard guard(q.device());
   at::Tensor o;
-  if constexpr (SPLIT) {
-    const at::NoGradGuard no_grad;
-    o = split_kv_forward(q, k, v, causal != 0, scale).first;
-  } else {
-    o = FlashAttention::apply(q, k, v, causal != 0, scale);
+  {
+    // Allocations and launches may block (a full launch queue, a cudaMalloc), and a host callback of the stream may
+    // need the GIL before the queue moves on.
+    const pybind11::gil_scoped_release no_gil;
+    const c10::cuda::OptionalCUDAGuard guard(q.device());
+    if constexpr (SPLIT) {
+      const at::NoGradGuard no_grad;
+      o = split_kv_forward(q, k, v, causal != 0, scale).first;
+    } else {
+      o = FlashAttention::apply(q, k, v, causal != 0, scale);
+    }
   }
   return THPVariable_Wrap(std::move(o));
   END_HANDLE_TH_ERRORS
@@ -294,8 +299,8 @@ PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* paged(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n != 8 || !plain_tensors(args, 5) || !ordinary_mode()) Py_RETURN_NONE;
-  const at::Tensor &q = THPVariable_Unpack(args[0]), &kc = THPVariable_Unpack(args[1]), &vc = THPVariable_Unpack(args[2]),
-                   &lens = THPVariable_Unpack(args[3]), &tables = THPVariable_Unpack(args[4]);
+  const at::Tensor q = THPVariable_Unpack(args[0]), kc = THPVariable_Unpack(args[1]), vc = THPVariable_Unpack(args[2]),
+                   lens = THPVariable_Unpack(args[3]), tables = THPVariable_Unpack(args[4]);
   if (!ready(q, 3) || !ready(kc, 4) || !ready(vc, 4)) Py_RETURN_NONE;
   const auto dt = q.scalar_type();
   if ((dt != at::kHalf && dt != at::kBFloat16) || kc.scalar_type() != dt || vc.scalar_type() != dt ||
@@ -319,34 +324,38 @@ PyObject* paged(PyObject*, PyObject* const* args, Py_ssize_t n) {
     PyErr_Clear();
     Py_RETURN_NONE;
   }
-  const c10::cuda::OptionalCUDAGuard guard(q.device());
-  const at::NoGradGuard no_grad;
-  const int64_t seqs = q.size(0), H = q.size(1), D = q.size(2), rows = seqs * H;
-  const int64_t S = asked > 0 ? asked : api.splitkv_num_splits(seqs, H, kc.size(1), 1, longest, D, sm_count(q));
-  at::Tensor out = at::empty({seqs, H, D}, q.options());
-  at::Tensor parts = at::empty({rows * (S * D + S + 1)}, q.options().dtype(at::kFloat));
-  b200attn_paged_params p{};
-  auto rows4 = [](const at::Tensor& t) {  // [seqs, heads, D] described as [seqs, heads, 1, D]
-    b200attn_tensor r;
-    r.ptr = t.data_ptr();
-    r.stride[0] = t.stride(0); r.stride[1] = t.stride(1); r.stride[2] = t.size(2); r.stride[3] = t.stride(2);
-    return r;
-  };
-  p.q = rows4(q); p.o = rows4(out);
-  p.key_cache = tensor4(kc); p.value_cache = tensor4(vc);
-  p.block_table = tables.data_ptr<int32_t>();
-  p.block_table_stride = tables.stride(0);
-  p.context_lens = lens.data_ptr<int32_t>();
-  p.part_o = parts.data_ptr<float>();
-  p.part_lse = p.part_o + rows * S * D;
-  p.lse = p.part_lse + rows * S;
-  p.num_seqs = seqs; p.Hq = H; p.Hkv = kc.size(1); p.D = D; p.block_size = kc.size(2); p.num_blocks = kc.size(0);
-  p.max_context_len = longest;
-  p.num_splits = S;
-  p.dtype = dtype_code(dt);
-  p.sm_scale = static_cast<float>(scale);
-  p.status = status_word(q.get_device());
-  check(api.paged(&p, current_stream(q)), "b200attn_paged_attention");
+  at::Tensor out;
+  {
+    const pybind11::gil_scoped_release no_gil;  // as above
+    const c10::cuda::OptionalCUDAGuard guard(q.device());
+    const at::NoGradGuard no_grad;
+    const int64_t seqs = q.size(0), H = q.size(1), D = q.size(2), rows = seqs * H;
+    const int64_t S = asked > 0 ? asked : api.splitkv_num_splits(seqs, H, kc.size(1), 1, longest, D, sm_count(q));
+    out = at::empty({seqs, H, D}, q.options());
+    at::Tensor parts = at::empty({rows * (S * D + S + 1)}, q.options().dtype(at::kFloat));
+    b200attn_paged_params p{};
+    auto rows4 = [](const at::Tensor& t) {  // [seqs, heads, D] described as [seqs, heads, 1, D]
+      b200attn_tensor r;
+      r.ptr = t.data_ptr();
+      r.stride[0] = t.stride(0); r.stride[1] = t.stride(1); r.stride[2] = t.size(2); r.stride[3] = t.stride(2);
+      return r;
+    };
+    p.q = rows4(q); p.o = rows4(out);
+    p.key_cache = tensor4(kc); p.value_cache = tensor4(vc);
+    p.block_table = tables.data_ptr<int32_t>();
+    p.block_table_stride = tables.stride(0);
+    p.context_lens = lens.data_ptr<int32_t>();
+    p.part_o = parts.data_ptr<float>();
+    p.part_lse = p.part_o + rows * S * D;
+    p.lse = p.part_lse + rows * S;
+    p.num_seqs = seqs; p.Hq = H; p.Hkv = kc.size(1); p.D = D; p.block_size = kc.size(2); p.num_blocks = kc.size(0);
+    p.max_context_len = longest;
+    p.num_splits = S;
+    p.dtype = dtype_code(dt);
+    p.sm_scale = static_cast<float>(scale);
+    p.status = status_word(q.get_device());
+    check(api.paged(&p, current_stream(q)), "b200attn_paged_attention");
+  }
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
 }

@@ -1,9 +1,13 @@
 """The native host path against the Python one it stands in front of: same results for every form that it takes, and every
 other form handed on (copies, wrong arguments, transforms)."""
+import sys
+import threading
+import time
+
 import pytest
 import torch
 
-from flagattention_b200 import _lib, flash_attention, flash_attention_split_kv, paged_attention
+from flagattention_b200 import _lib, flash_attention, flash_attention_split_kv, paged_attention, status
 from gpu_util import device, make_qkv
 
 pytestmark = pytest.mark.gpu
@@ -112,6 +116,44 @@ def test_gradient_of_another_type_stride_and_only_some_inputs():
     c, = torch.autograd.grad(o.float().sum(), k)        # an expanded gradient
     d, = torch.autograd.grad(flash_attention(q, k, v), k, torch.ones_like(o))
     assert torch.equal(c, d)
+
+
+@pytest.mark.parametrize("call", ["flash", "split_kv", "paged"])
+def test_other_threads_run_while_a_call_waits(call, monkeypatch):
+    """A call that has to wait for room in the launch queue does not hold the GIL. With a switch interval far beyond the
+    test's length another thread gets it only from a call that lets go of it (the status poll, which would, is put off)."""
+    q, k, v, _ = make_qkv(2, 4, 2, 64, 64, 64, torch.float16, seed=1)
+    q1 = q[:, :, 0].contiguous()
+    lens, tables = torch.tensor([40, 64], device=device(), dtype=torch.int32), torch.zeros(2, 4, device=device(), dtype=torch.int32)
+    cache = torch.randn(3, 2, 16, 64, device=device(), dtype=torch.float16)
+    host = _lib.host()
+    run = {"flash": lambda: host.flash(q, k, v, False, None), "split_kv": lambda: host.split_kv(q, k, v, False, None),
+           "paged": lambda: host.paged(q1, cache, cache, lens, tables, 0.125, 64, 0)}[call]
+    assert run() is not None
+    status.check_device_status(device())
+    monkeypatch.setattr(status, "POLL_INTERVAL_S", float("inf"))
+    turns, stop = [0], threading.Event()
+
+    def other():
+        while not stop.is_set():
+            turns[0] += 1
+            time.sleep(0.001)
+    interval = sys.getswitchinterval()
+    thread = threading.Thread(target=other)
+    sys.setswitchinterval(1000.0)
+    try:
+        thread.start()
+        torch.cuda._sleep(int(3e8))   # about 0.15 s on the device, in which the queue fills up
+        before = turns[0]
+        for _ in range(3000):
+            run()
+        got = turns[0] - before
+    finally:
+        stop.set()
+        sys.setswitchinterval(interval)
+        thread.join()
+        torch.cuda.synchronize()
+    assert got > 10
 
 
 def test_saved_tensor_hooks_see_what_is_kept():
