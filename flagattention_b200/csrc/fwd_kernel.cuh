@@ -204,7 +204,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     int n_sub[2];    // SPLIT64: number of 64-key sub-steps each query tile runs
     int n_max;       // number of K/V tiles the CTA streams
   };
-  bool longest_first = false;  // sort_entries, and the sequences differ in length
   auto get_item = [&](int id) -> Item {
     Item it;
     const BlockCoord bc = args.order.decode(id);
@@ -212,8 +211,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     it.split = bc.z - z_row * args.num_splits;
     const int m_blk = args.div_splits.div(args.n_zblocks) - 1 - z_row;  // longest first
     it.b = args.div_heads.div(bc.bh);
-    const int head = longest_first ? id % grid_heads : bc.bh - it.b * grid_heads;
-    if (longest_first) {
+    const int head = args.sort_entries > 0 ? id % grid_heads : bc.bh - it.b * grid_heads;
+    if (args.sort_entries > 0) {
       it.b = *my_entry / args.num_splits;
       it.split = *my_entry - it.b * args.num_splits;
     }
@@ -303,8 +302,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
       tiles[e] = mine;
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the Q tile is loaded over `tiles`
-    longest_first = __syncthreads_or(differs);
-    if (longest_first) {
+    if (threadIdx.x == 0) *my_entry = static_cast<int>(blockIdx.x) / grid_heads;  // (equal lengths: as given)
+    if (__syncthreads_or(differs)) {
       if (e < n) {
         int rank = 0;
         for (int j = 0; j < n; ++j) {
