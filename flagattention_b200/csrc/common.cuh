@@ -195,10 +195,10 @@ __device__ __forceinline__ uint32_t keep_mask_one(uint32_t word, int i) {
 // Keep decisions of 32 consecutive counters base, base+1, ..., base+31 as a word in the order above. The
 // counter's high word is the same for all 32 unless the low word wraps inside the run, so everything that depends
 // on it is prepared once, the first round's product advances by a constant, and the remaining rounds are written out
-// with the product halves that reach output word 0. The fold and the comparison are one range test (dropped
-// means -T - 1 <= x <= T) whose carry is shifted into the word. Measured at full occupancy: 950 G draws/s against
-// 834 for the loop over philox6_word0() with fold, compare and insert; forming the high halves on the double-precision
-// pipe instead (2^84 + a * b rounded down to multiples of 2^32) measured 600 to 970 and is not used.
+// with the product halves that reach output word 0. The fold and the comparison are one range test (kept means
+// x + T + 1 > 2 T + 1 as unsigned numbers) whose carry is shifted into the word. keep_mask_kernel takes 1.25 ms for 2^30
+// decisions (858 G/s), and 1.38 with the loop over philox6_word0() with fold, compare and insert; forming the high halves on
+// the double-precision pipe (2^84 + a * b rounded down to multiples of 2^32) measured 0.6 to 1.02 of the rate and is not used.
 __device__ __forceinline__ uint32_t dropout_keep_word(const DropoutCtx& c, uint64_t base) {
   constexpr uint32_t KEY_A = 0x9E3779B9u, KEY_B = 0xBB67AE85u;
   constexpr uint32_t ROUND_A = 0xD2511F53u, ROUND_B = 0xCD9E8D57u;
@@ -213,7 +213,7 @@ __device__ __forceinline__ uint32_t dropout_keep_word(const DropoutCtx& c, uint6
     const uint32_t kb3 = static_cast<uint32_t>(second) ^ (c.seed_hi + 2 * KEY_B);
     const uint32_t kb4 = c.seed_hi + 3 * KEY_B, kb5 = c.seed_hi + 4 * KEY_B;
     const uint32_t shift = static_cast<uint32_t>(c.keep_threshold) + 1u;
-    const uint32_t span = 2u * static_cast<uint32_t>(c.keep_threshold) + 1u;
+    const uint32_t above = ~(2u * static_cast<uint32_t>(c.keep_threshold) + 1u);  // x + shift + above carries: kept
 #pragma unroll
     for (int bit = 31; bit >= 0; --bit) {
       // words 0 and 2 after round r: xr, yr
@@ -229,10 +229,8 @@ __device__ __forceinline__ uint32_t dropout_keep_word(const DropoutCtx& c, uint6
       const uint32_t y4 = static_cast<uint32_t>(q4 >> 32) ^ static_cast<uint32_t>(q3) ^ kb4;
       const uint32_t y5 = __umulhi(ROUND_A, x4) ^ static_cast<uint32_t>(q4) ^ kb5;
       const uint32_t x6 = __umulhi(ROUND_B, y5) ^ (ROUND_B * y4) ^ ka6;
-      uint32_t rest;
-      asm("sub.cc.u32 %0, %2, %3;\n\taddc.u32 %1, %1, %1;" : "=r"(rest), "+r"(bits) : "r"(span), "r"(x6 + shift));
+      asm("{\n\t.reg .u32 sum;\n\tadd.cc.u32 sum, %1, %2;\n\taddc.u32 %0, %0, %0;\n\t}" : "+r"(bits) : "r"(x6 + shift), "r"(above));
     }
-    bits = ~bits;
   } else {
 #pragma unroll 1
     for (int i = 0; i < 32; ++i) bits |= (dropout_keep(c, base + i) ? 1u : 0u) << keep_bit_of(i);
