@@ -96,6 +96,11 @@ __global__ void dq_convert_kernel(const float* __restrict__ acc, uint16_t* __res
 // is in steps of 64 queries: a block's start-up, its fp32 sums and their exchange cost about `fixed` steps.
 // Training step with one block -> shared key blocks, replayed from a graph, D = 128 bf16: B2 Hq8 Hkv2 512 causal
 // 67 -> 46 us, B1 Hq8 Hkv2 1024 causal 114 -> 54, B2 Hq32 Hkv4 1024 without a mask 234 -> 164.
+// The number depends on how many (batch, KV head) pairs the call has, and with it the order in which the fp32 sums of dK and
+// dV are formed. A number from the shape alone costs where the chip is full: at D = 128 two blocks per key block take 724 ->
+// 974 us at 444 pairs of 4 heads x 512 keys, 973 -> 1292 at 222 pairs x 1024, and only from some 512 steps on less than 3 %.
+// (At D = 64 and 32 it counts the two resident blocks of the fused pass for the separate kernels of deterministic mode
+// too, so that both modes give the same dK and dV.)
 static int bwd_kv_split(const BwdArgs& a, int D) {
   const int n_z = a.n_zblocks;
   const int64_t pairs = static_cast<int64_t>(a.B) * a.Hkv;
@@ -110,8 +115,8 @@ static int bwd_kv_split(const BwdArgs& a, int D) {
     sum += steps;
     if (steps > longest) longest = steps;
   }
-  // Long key blocks keep one block each, so that a call over some of the (batch, KV head) pairs gives the bits of
-  // the whole call.
+  // Long key blocks keep one block each: over long sequences a call on some of the (batch, KV head) pairs gives the
+  // bits of the whole call (sharding.py), whatever their number.
   if (longest > 128) return 1;
   int best = 1;
   double best_time = 0.;
@@ -262,6 +267,18 @@ static int run_total(const b200attn_total_params* p, float2* stats, cudaStream_t
 }
 
 }  // namespace b200attn
+
+extern "C" int32_t b200attn_bwd_key_block_split(int32_t B, int32_t Hq, int32_t Hkv, int32_t M, int32_t N, int32_t D,
+                                                int32_t causal) {
+  using namespace b200attn;
+  if (check_common("bwd_key_block_split", B, Hq, Hkv, M, N, D, B200ATTN_F16) != B200ATTN_OK) return 0;
+  BwdArgs a{};
+  a.B = B; a.Hq = Hq; a.Hkv = Hkv; a.M = M; a.N = N;
+  a.groups = Hq / Hkv;
+  a.n_zblocks = cdiv(N, 128);
+  a.causal = fold_band(causal != 0, 0, 0, 0, &a.d_min, &a.d_max) ? 1 : 0;
+  return bwd_kv_split(a, D);
+}
 
 extern "C" size_t b200attn_bwd_workspace_bytes(int32_t B, int32_t Hq, int32_t Hkv, int32_t M, int32_t N,
                                                int32_t D) {

@@ -4,8 +4,15 @@ The operator is independent per (batch, KV head): all query heads that share a K
 rank, so dK/dV need no cross-rank reduction. ``unit_range`` assigns each rank a contiguous range
 of the ``B * Hkv`` units; ``shard`` returns the matching views of q, k, v (and anything shaped
 like q), one piece per batch the range touches. One process per GPU runs its pieces through the
-ordinary ``flash_attention``; results are bit-identical to the corresponding slices of a
-single-GPU run.
+ordinary ``flash_attention``.
+
+Outputs are bit-identical to the corresponding slices of a single-GPU run, unless the piece has so few
+query rows that the forward splits its keys (``split_kv.choose_num_splits``, which counts batch and heads).
+So are dK and dV when the backward shares its key blocks between as many thread blocks for the piece as for
+the whole (``b200attn_bwd_key_block_split`` of the C ABI tells; long sequences, more than 128 steps of 64
+queries by the query heads of a KV head, never share): otherwise they agree to the order of fp32 sums before
+one rounding. dQ at head dimensions 32 and up is summed in no fixed order by default; under
+``torch.use_deterministic_algorithms(True)`` it is bit-identical like the outputs, given the same outputs.
 """
 from __future__ import annotations
 

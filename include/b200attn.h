@@ -145,6 +145,12 @@ size_t b200attn_bwd_workspace_bytes(int32_t B, int32_t Hq, int32_t Hkv, int32_t 
                                     int32_t D);
 int b200attn_bwd(const b200attn_bwd_params* p, void* stream);
 
+/* How many thread blocks share the queries of one 128-key block in the dK/dV pass of such a call on the current device
+ * (1: none; 0: a bad argument). With few key blocks they are shared by up to eight, whose fp32 partial sums are added in a
+ * fixed order: two calls on the same data with the same number give the same bits of dK and dV, with another number they
+ * agree to the order of fp32 sums. Key blocks of more than 128 steps (64 queries of one head each) are never shared. */
+int32_t b200attn_bwd_key_block_split(int32_t B, int32_t Hq, int32_t Hkv, int32_t M, int32_t N, int32_t D, int32_t causal);
+
 /* The same backward restricted to some of its stages, so a profiler or benchmark can time the
  * kernels one by one. PREP = delta + statistics preprocess, KV = the dK/dV kernel, Q = the dQ
  * kernel; KV and Q need the scratch PREP wrote. At D >= 32 the KV stage is a fused pass that also

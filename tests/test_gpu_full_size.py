@@ -4,7 +4,8 @@ The oracle cannot materialise whole score matrices at these sizes, so each confi
 through (a) the oracle on a slice that is independent of the rest (one batch / KV group, or a band
 of query rows with the keys it can see) and (b) size-independent properties: rows of P sum to one,
 total attention sums to the number of queries, shard-by-head results are bit-identical to the
-corresponding slice of the full run, repeated runs are bit-identical."""
+corresponding slice of the full run (at these lengths the backward shares no key blocks), repeated runs are
+bit-identical."""
 import math
 
 import pytest
@@ -54,7 +55,7 @@ def test_c2_gqa_prefill_train_step():
     g2 = torch.autograd.grad(o2, (q2, k2, v2), dos.clone(), retain_graph=True)
     assert torch.equal(o2, o[b:b + 1, 4 * g:4 * g + 4]) and torch.equal(lse2, lse[b:b + 1, 4 * g:4 * g + 4])
     assert torch.equal(g2[1], dk[b:b + 1, g:g + 1]) and torch.equal(g2[2], dv[b:b + 1, g:g + 1])
-    # dQ at D = 128 and 64 is summed over the key blocks by fp32 reductions whose order is not fixed: equal up
+    # dQ at D >= 32 is summed over the key blocks by fp32 reductions whose order is not fixed: equal up
     # to that, and bit for bit when PyTorch's deterministic mode selects the two separate kernels.
     torch.testing.assert_close(g2[0].float(), dq[b:b + 1, 4 * g:4 * g + 4].float(), atol=2e-3, rtol=2e-2)
     torch.use_deterministic_algorithms(True)
