@@ -36,8 +36,8 @@
 // one block spend half their time on their own latencies, and with short sequences a block's start-up, first loads and
 // output stores weigh as much as its steps; a second block fills both. Each has half the TMEM, which leaves one
 // (T1, T2) buffer, so its steps are serial. Measured, one block per SM -> two: training step B64 H32 512 x 512 D64
-// causal fp16 (forward included) 1105 -> 945 us, B16 H16 2048 x 2048 D64 with dropout 4085 -> 3590 us; at D = 32, two
-// separate passes -> this one: B2 H16 4096 x 4096 causal bf16 455 -> 387 us.
+// causal fp16 (forward included) 1105 -> 892 us, B16 H16 2048 x 2048 D64 with dropout 4110 -> 3645 us; at D = 32, two
+// separate passes -> this one: B2 H16 4096 x 4096 causal bf16 455 -> 387 us. (80 registers a thread, 14 to 30 bytes spilled.)
 //
 // Per-query statistics come from a padded scratch array holding, per pair of queries, the float4
 // (-lse[m]*log2e, -lse[m+1]*log2e, -delta[m], -delta[m+1]); it is padded to a multiple of 128
@@ -80,7 +80,7 @@ struct BwdSmem {
   static constexpr int STAGES = DUO ? 2 : (FUSED && D == 128) ? 3 : 4;
   static constexpr int NBUF = DUO ? 1 : 2;                     // (T1, T2) buffers
   // Total attention has one product and one exponential per score and no accumulator: two blocks fit and fill each
-  // other's waits (training step with dropout and both auxiliary outputs, B16 H16 2048 x 2048 D64: 3610 -> 3465 us).
+  // other's waits (training step with dropout and both auxiliary outputs, B16 H16 2048 x 2048 D64: 3645 -> 3483 us).
   static constexpr int BLOCKS = DUO || MODE == MODE_TOTAL ? 2 : 1;
   static constexpr int TMEM_COLS = 512 / BLOCKS;
   static constexpr int N_A = MODE == MODE_TOTAL ? 1 : 2;       // resident tiles

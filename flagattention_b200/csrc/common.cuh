@@ -56,9 +56,12 @@ inline int launch(const LaunchForm& form, void (*kernel)(Params...), dim3 grid, 
   return B200ATTN_OK;
 }
 // The forward and decode kernels and the combine step of split keys are short enough for the gap between two launches
-// to show, and are launched chained: B1 H4 128 x 128 D64 forward 5.7 -> 4.8 us a call replayed from a graph, paged
-// decode of 32 sequences up to 4096 keys 95.4 -> 92.8 us. The backward's kernels are not: chained, its dK/dV pass runs
+// to show, and are launched chained: B1 H4 128 x 128 D64 forward 6.5 -> 5.5 us a call replayed from a graph, paged
+// decode of 32 sequences up to 4096 keys 96 -> 92 us. The backward's kernels are not: chained, its dK/dV pass runs
 // beside the waiting blocks of the dQ conversion, and a step of B64 H32 512 x 512 D64 took 817 instead of 796 us.
+// Not every launch gains (replayed from a graph, plain -> chained): decode of two rows per KV head, B2 Hq16 Hkv8 3001 keys,
+// 13.4 -> 17.1 us, B16 H8 500 D64 7.6 -> 8.9; B2 H16 8192 36.9 -> 36.2, B4 Hq16 Hkv8 1000 D64 8.6 -> 8.1; paged H8 11401 D64,
+// two sequences, 16.9 -> 15.8; back to back from Python the small ones are bound by the host either way.
 constexpr LaunchForm CHAINED{true, 1};
 
 // One-time set-up per device (kernel attributes, device properties) that any host thread may

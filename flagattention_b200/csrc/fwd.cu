@@ -100,9 +100,10 @@ static int run_fwd(const b200attn_fwd_params* p, const float* merge_o, const flo
   }
   // D <= 64 with 16-bit output: one query tile per block, four blocks per SM (fwd_solo.cuh), where there is a mask or
   // the sequences are short. Forward, two tiles -> one: B4 Hq32 Hkv8 4096 causal D64 bf16 430 -> 375 us, 16384 causal
-  // 732 -> 708, B64 H32 512 causal (training step) 982 -> 820; 4096 without a mask 717 -> 726, so long launches without a
-  // mask keep the pairs, whose shared K/V tiles then pay. At D = 128 (two blocks per SM) it lost everywhere (B4 Hq16
-  // 2048 causal 82 -> 93 us).
+  // 732 -> 708, B64 H32 512 causal 265 -> 174, 128 without a mask 64 -> 31; at D = 32 512 causal 230 -> 148, 128 causal 63
+  // -> 27; at D = 16 B16 H32 1024 causal 147 -> 108; D64 4096 without a mask 717 -> 726, so long launches without a mask
+  // keep the pairs, whose shared K/V tiles then pay. At D = 128 (two blocks per SM) it lost everywhere (B4 Hq16 2048 causal
+  // 82 -> 93 us).
   L.solo = p->D <= 64 && L.args.o_tma && merge_o == nullptr && (fold_band(p->causal != 0, p->band, p->dist_min, p->dist_max, &band_lo, &band_hi) ||
                                           p->N <= 1024) &&
            static_cast<int64_t>(p->B) * p->Hq * cdiv(p->M, 128) <= 2147483647ll;
