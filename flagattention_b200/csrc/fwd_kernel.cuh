@@ -211,8 +211,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     it.split = bc.z - z_row * args.num_splits;
     const int m_blk = args.div_splits.div(args.n_zblocks) - 1 - z_row;  // longest first
     it.b = args.div_heads.div(bc.bh);
-    const int head = args.sort_entries > 0 ? id % grid_heads : bc.bh - it.b * grid_heads;
-    if (args.sort_entries > 0) {
+    const bool sorted = !SPLIT64 && args.sort_entries > 0;  // (the 64-key pipeline never serves a paged cache)
+    const int head = sorted ? id % grid_heads : bc.bh - it.b * grid_heads;
+    if (sorted) {
       it.b = *my_entry / args.num_splits;
       it.split = *my_entry - it.b * args.num_splits;
     }
@@ -288,7 +289,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
   const uint32_t tmem_base = *tmem_slot;
   pdl_trigger();
   pdl_wait();
-  if (args.sort_entries > 0) {
+  if (!SPLIT64 && args.sort_entries > 0) {
     // Blocks id, id + 1, ... take the heads of the longest entry, then of the next: thread t ranks entry t.
     int* tiles = reinterpret_cast<int*>(sQ);  // (no load has been issued yet)
     const int e = static_cast<int>(threadIdx.x), n = args.sort_entries;
