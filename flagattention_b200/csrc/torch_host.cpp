@@ -68,6 +68,19 @@ int32_t* status_word(int device) {
   return word;
 }
 
+// Lets go of the GIL. (pybind11::gil_scoped_release also looks up and updates its own thread state, a part of a
+// microsecond that shows in a call of five.)
+class NoGil {
+ public:
+  NoGil() : state_(PyEval_SaveThread()) {}
+  ~NoGil() { PyEval_RestoreThread(state_); }
+  NoGil(const NoGil&) = delete;
+  NoGil& operator=(const NoGil&) = delete;
+
+ private:
+  PyThreadState* state_;
+};
+
 // A plain strided CUDA tensor of `dims` dimensions that TMA can describe as it is.
 bool ready(const at::Tensor& x, int dims) {
   using c10::DispatchKey;
@@ -282,7 +295,7 @@ PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
   {
     // Allocations and launches may block (a full launch queue, a cudaMalloc), and a host callback of the stream may
     // need the GIL before the queue moves on.
-    const pybind11::gil_scoped_release no_gil;
+    const NoGil no_gil;
     const c10::cuda::OptionalCUDAGuard guard(q.device());
     if constexpr (SPLIT) {
       const at::NoGradGuard no_grad;
@@ -326,7 +339,7 @@ PyObject* paged(PyObject*, PyObject* const* args, Py_ssize_t n) {
   }
   at::Tensor out;
   {
-    const pybind11::gil_scoped_release no_gil;  // as above
+    const NoGil no_gil;  // as above
     const c10::cuda::OptionalCUDAGuard guard(q.device());
     const at::NoGradGuard no_grad;
     const int64_t seqs = q.size(0), H = q.size(1), D = q.size(2), rows = seqs * H;
